@@ -12,7 +12,7 @@
 // signals "operands ready" on an mbarrier and waits on its "done" mbarrier
 // (tcgen05.commit). For each tile, entirely on chip:
 //   encode the input rows into a BF16/FP16 operand tile (A0)
-//   forward:  h0 = relu(A0 W0^T), h1, h2 (kept in shared memory), raw = h2 W3^T
+//   forward:  h0 = relu(A0 W0^T), h1, h2 (h0 and h1 parked in TMEM), raw = h2 W3^T
 //   adjoint:  KL loss and dL/draw per record in registers (train.cu:69-124)
 //   backward: for l = 3..0
 //               weight gradient  dW_l += delta_l^T h_{l-1}   (M = 64, MN-major
@@ -27,9 +27,9 @@
 // global gradient. Adam + EMA then run as one streaming kernel.
 //
 // TMEM (512 columns): one forward/data-gradient accumulator per pipeline
-// (M = 128; 64 columns, 128 when the output layer is wider), then the shared
-// weight-gradient accumulators dW0 | dW1 | dW2 | dW3^T (M = 64: rows live in
-// lanes 0-15 of each 32-lane subpartition). The layer-0 data gradient is
+// (M = 128; 64 columns, 80 for 16 lobes), then the shared weight-gradient
+// accumulators dW0 | dW1 | dW2 | dW3^T (M = 64: rows live in lanes 0-15 of
+// each 32-lane subpartition), then the parked activations (TrainShape). The layer-0 data gradient is
 // computed for the grid columns only, the only ones with parameters below.
 //
 // Gradient scale: delta is the reference's loss_scale/n scaled gradient
@@ -105,6 +105,14 @@ NMG_D void load_chunk(const uint8_t* tile, int row, int chunk, int chunks, float
   f[7] = p.y;
 }
 
+// Half h of 16-bit row `row` of a 64-column tile from its 16 packed words.
+NMG_D void store_half_row(uint8_t* tile, int row, int h, const uint32_t (&pk)[16]) {
+#pragma unroll
+  for (int c = 0; c < kWidth / 16; ++c)
+    *reinterpret_cast<uint4*>(tile + tc::cm_offset(row, h * (kWidth / 16) + c, kWidth / 8)) =
+        make_uint4(pk[4 * c], pk[4 * c + 1], pk[4 * c + 2], pk[4 * c + 3]);
+}
+
 // Number of tiles warpgroup g of this CTA processes (the same expression in
 // the compute warpgroups and in the MMA issuer).
 NMG_D int wg_tiles(int ntiles, int g, int nwg) {
@@ -171,9 +179,9 @@ NMG_D void scatter_level(const FusedArgs& a, float* gt, int lv, const float (&p3
 // Scatter warps (SCAT): the CTA adds 7 warps (with the issuer warp they form
 // two more warpgroups) that apply each tile's grid gradient to the table
 // while the pipelines move on to their next tile. A pipeline stages its
-// layer-0 data gradient in its third hidden tile (dead by then, rewritten
-// only at the next tile's third forward layer) and arrives on sfull; the
-// scatter warps arrive on sempty when they have read it.
+// layer-0 data gradient in its delta tile (dead by then, rewritten only at
+// the next tile's loss) and arrives on sfull; the scatter warps arrive on
+// sempty when they have read it.
 // Registers: the 768-thread block launches at 80 per thread and moves 32 of
 // them from each issuer/scatter thread to the compute threads.
 constexpr int kScatThreadsPerCta = 6 * kRows;
@@ -181,35 +189,71 @@ constexpr int kScatRegLaunch = 80, kScatRegCompute = 96, kScatRegScatter = 48;
 static_assert(4 * kRows * kScatRegCompute + 2 * kRows * kScatRegScatter == kScatThreadsPerCta * kScatRegLaunch,
               "register split must equal the launch allocation");
 
+// A pipeline's shared memory and the CTA's TMEM columns. A hidden layer's
+// activations are needed twice, as the next layer's operand and again in the
+// backward pass; between the two they are parked in TMEM (packed, 32 columns
+// a layer), so that a pipeline holds one hidden tile (two where the output
+// layer leaves room to park one layer only) instead of three. That matters
+// because the gathers live on what shared memory leaves of the SM's 256 KB
+// to L1: every sector in flight holds a 128-byte line, and 28 KB of L1 (three
+// hidden tiles and a separate delta tile) kept the gathers at ~0.33 sectors
+// per cycle; with 92 KB (148 KB of shared memory at 8 lobes) a 2^18-record
+// batch takes 259 us instead of 292 us, the training step 434 instead of
+// 468 us (2^16 records on FP16: 277 instead of 298 us).
+template <int F, int LEVELS, int MODE, int SHDEG, int BINS, int NOUTMAX, int NWG, bool SCAT, bool REC>
+struct TrainShape {
+  static constexpr int NDIR = MODE == 0 ? SHDEG * SHDEG + 3 * BINS : 2 * SHDEG * SHDEG + BINS;
+  static constexpr int NENC = (LEVELS * F + NDIR + 15) / 16 * 16;
+  static constexpr int NGRID = LEVELS * F;
+  static constexpr int DMAX = NOUTMAX > kWidth ? NOUTMAX : kWidth;
+  // TMEM: one forward/data-gradient accumulator per pipeline (a hidden
+  // layer's 64 columns or the output layer's NOUTMAX), the shared
+  // weight-gradient accumulators (M = 64) dW0 | dW1 | dW2 | dW3^T, then the
+  // parked activations.
+  static constexpr uint32_t DCOLS = NOUTMAX <= kWidth ? kWidth : (NOUTMAX + 15) / 16 * 16;
+  static constexpr uint32_t CW0 = NWG * DCOLS, CW1 = CW0 + NENC, CW2 = CW1 + kWidth, CW3 = CW2 + kWidth;
+  static constexpr uint32_t CPK = CW3 + (NOUTMAX + 15) / 16 * 16;
+  static constexpr int PARK = CPK + 2 * NWG * (kWidth / 2) <= kTrainCols ? 2 : 1;  // layers parked: h0, h1 or h0
+  static_assert(CPK + PARK * NWG * (kWidth / 2) <= kTrainCols, "TMEM holds 512 columns");
+  static constexpr int NH = 3 - PARK;  // hidden tiles
+  static constexpr uint32_t A_BYTES = kRows * NENC * 2;
+  static constexpr uint32_t H_BYTES = kRows * kWidth * 2;
+  static constexpr uint32_t D_BYTES = kRows * DMAX * 2;
+  static constexpr uint32_t DGS_BYTES = NGRID * kRows * 4;  // the grid gradient staged in the delta tile
+  static_assert(DGS_BYTES <= D_BYTES, "grid gradient staging fits the delta tile");
+  // after the operand tiles: each row's GuidedOutput (records mode: computed
+  // at the load stage, read before the loss stage writes the delta tile; at
+  // the delta tile's end where the staged grid gradient leaves room), by tile
+  // parity each row's normalised position for the scatter warps, and the
+  // loss's partial sums of both halves of each row
+  static constexpr uint32_t ROW_BYTES = kRows * 8 * 4;
+  static constexpr bool REC_IN_D = D_BYTES >= DGS_BYTES + ROW_BYTES;
+  static constexpr uint32_t REC_BYTES = REC && !REC_IN_D ? ROW_BYTES : 0, P3_BYTES = SCAT ? 2 * kRows * 4 * 4 : 0;
+  static constexpr uint32_t XCH_BYTES = 2 * kRows * 2 * 4;
+  static constexpr uint32_t D_OFF = A_BYTES + NH * H_BYTES, P3_OFF = D_OFF + D_BYTES + REC_BYTES;
+  static constexpr uint32_t REC_OFF = D_OFF + (REC_IN_D ? DGS_BYTES : D_BYTES);
+  static constexpr uint32_t WG_BYTES = P3_OFF + P3_BYTES + XCH_BYTES;
+  // offset of h_l's tile in the forward pass, and of h_l's (then delta_l's,
+  // which replaces it in place) in the backward pass; delta_3 is the delta tile
+  NMG_HD static uint32_t fwd_off(int l) { return A_BYTES + (NH == 2 && l == 1 ? H_BYTES : 0u); }
+  NMG_HD static uint32_t bwd_off(int l) {
+    if (l == 3) return D_OFF;
+    return l == 1 ? (NH == 2 ? A_BYTES + H_BYTES : D_OFF) : A_BYTES;
+  }
+  static size_t smem_bytes(uint32_t w_bytes) { return size_t((w_bytes + 1023u) & ~1023u) + NWG * size_t(WG_BYTES) + 256; }
+};
+
 template <int F, int LEVELS, int MODE, int SHDEG, int BINS, int K, int NOUTMAX, bool SMOOTH, int NWG, bool SCAT,
           bool REC>
 __global__ void __launch_bounds__(SCAT ? kScatThreadsPerCta : 2 * NWG * kRows + 32, 1)
     k_fused_train(const __grid_constant__ TrainArgs ta) {
   static_assert(!SCAT || NWG == 2, "scatter warps pair with two pipelines");
   static_assert(K % 8 == 0, "each half of a row holds K / 2 lobes, a whole number of 16-column groups");
-  constexpr int NDIR = MODE == 0 ? SHDEG * SHDEG + 3 * BINS : 2 * SHDEG * SHDEG + BINS;
-  constexpr int NENC = (LEVELS * F + NDIR + 15) / 16 * 16;
-  constexpr int NGRID = LEVELS * F;
-  constexpr int DMAX = NOUTMAX > kWidth ? NOUTMAX : kWidth;
-  constexpr uint32_t A_BYTES = kRows * NENC * 2;
-  constexpr uint32_t H_BYTES = kRows * kWidth * 2;
-  constexpr uint32_t D_BYTES = kRows * DMAX * 2;
-  // per pipeline, after its operand tiles: each row's GuidedOutput (records
-  // mode REC: computed at the load stage, read at the loss stage), by tile
-  // parity each row's normalised position for the scatter warps, and the
-  // loss's partial sums of both halves of each row
-  constexpr uint32_t REC_BYTES = REC ? kRows * 8 * 4 : 0, P3_BYTES = SCAT ? 2 * kRows * 4 * 4 : 0;
-  constexpr uint32_t XCH_BYTES = 2 * kRows * 2 * 4;
-  constexpr uint32_t WG_BYTES = A_BYTES + 3 * H_BYTES + D_BYTES + REC_BYTES + P3_BYTES + XCH_BYTES;
+  using Sh = TrainShape<F, LEVELS, MODE, SHDEG, BINS, NOUTMAX, NWG, SCAT, REC>;
+  constexpr int NENC = Sh::NENC, NGRID = Sh::NGRID, PARK = Sh::PARK;
+  constexpr uint32_t WG_BYTES = Sh::WG_BYTES, DCOLS = Sh::DCOLS;
+  constexpr uint32_t CW0 = Sh::CW0, CW1 = Sh::CW1, CW2 = Sh::CW2, CW3 = Sh::CW3;
   constexpr int NL = 4;  // three hidden layers
-  // TMEM: one forward/data-gradient accumulator per pipeline, then the shared
-  // weight-gradient accumulators (M = 64) dW0 | dW1 | dW2 | dW3^T.
-  // (the accumulator holds a hidden layer's 64 columns or the output layer's
-  // NOUTMAX: 80 for 16 lobes, so that two pipelines and the weight gradients
-  // fit the 512 columns)
-  constexpr uint32_t DCOLS = NOUTMAX <= kWidth ? kWidth : (NOUTMAX + 15) / 16 * 16;
-  constexpr uint32_t CW0 = NWG * DCOLS, CW1 = CW0 + NENC, CW2 = CW1 + kWidth, CW3 = CW2 + kWidth;
-  static_assert(CW3 + NOUTMAX <= kTrainCols, "TMEM holds 512 columns");
   static_assert(NGRID <= 64 && NGRID % 16 == 0, "grid features are read in 16-column groups");
   extern __shared__ __align__(1024) uint8_t smem[];
   const FusedArgs& a = ta.f;
@@ -223,11 +267,10 @@ __global__ void __launch_bounds__(SCAT ? kScatThreadsPerCta : 2 * NWG * kRows + 
   const int t = threadIdx.x % kRows;                // row of the tile
   uint8_t* wsm = smem;
   uint8_t* A0 = smem + w_region + g * WG_BYTES;
-  uint8_t* Hs = A0 + A_BYTES;  // three hidden tiles
-  uint8_t* Dt = Hs + 3 * H_BYTES;
-  float* s_rec = reinterpret_cast<float*>(Dt + D_BYTES);             // [kRows][8]
-  float* s_p3 = reinterpret_cast<float*>(Dt + D_BYTES + REC_BYTES);  // [2][kRows][4]
-  float2* s_xch = reinterpret_cast<float2*>(Dt + D_BYTES + REC_BYTES + P3_BYTES);  // [2 halves][kRows]
+  uint8_t* Dt = A0 + Sh::D_OFF;
+  float* s_rec = reinterpret_cast<float*>(A0 + Sh::REC_OFF);                    // [kRows][8]
+  float* s_p3 = reinterpret_cast<float*>(A0 + Sh::P3_OFF);                      // [2][kRows][4]
+  float2* s_xch = reinterpret_cast<float2*>(A0 + Sh::P3_OFF + Sh::P3_BYTES);    // [2 halves][kRows]
   // [0] weights, then ready[], done[], sfull[], sempty[]
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + w_region + NWG * WG_BYTES);
   uint64_t* ready = bars + 1;
@@ -299,13 +342,12 @@ __global__ void __launch_bounds__(SCAT ? kScatThreadsPerCta : 2 * NWG * kRows + 
           last = clock64();
           tc::fence_after_sync();
           uint8_t* gA0 = smem + w_region + i * WG_BYTES;
-          uint8_t* gH = gA0 + A_BYTES;
-          uint8_t* gD = gH + 3 * H_BYTES;
+          const uint32_t g_addr = tc::smem_u32(gA0);
           const uint32_t tD = tbase + i * DCOLS;
           const int s = step[i];
           if (s < NL) {  // forward layer s
             const int kin = s == 0 ? NENC : kWidth;
-            const uint32_t a_addr = tc::smem_u32(s == 0 ? gA0 : gH + (s - 1) * H_BYTES);
+            const uint32_t a_addr = s == 0 ? g_addr : g_addr + Sh::fwd_off(s - 1);
             issue_mma_kmajor(tD, a_addr, kin / 8, w_addr + a.layer_off[s], 128u, uint32_t(kin / 8) * 128u, 256u,
                              s == NL - 1 ? nout : kWidth, kin / 16, fp16, false);
           } else {  // backward layer l: weight gradient then data gradient
@@ -313,17 +355,16 @@ __global__ void __launch_bounds__(SCAT ? kScatThreadsPerCta : 2 * NWG * kRows + 
             const int dchunks = l == NL - 1 ? KC3 : kWidth / 8;
             const int dwidth = l == NL - 1 ? nout : kWidth;
             const int in_w = l == 0 ? NENC : kWidth;
-            const uint8_t* hin = l == 0 ? gA0 : gH + (l - 1) * H_BYTES;
+            const uint32_t hin = l == 0 ? g_addr : g_addr + Sh::bwd_off(l - 1), del = g_addr + Sh::bwd_off(l);
             const bool acc = (started >> l) & 1u;
             if (l == NL - 1)
-              issue_wgrad(tbase + CW3, tc::smem_u32(hin), kWidth / 8, tc::smem_u32(gD), dchunks, dwidth, fp16, acc);
+              issue_wgrad(tbase + CW3, hin, kWidth / 8, del, dchunks, dwidth, fp16, acc);
             else
-              issue_wgrad(tbase + (l == 0 ? CW0 : (l == 1 ? CW1 : CW2)), tc::smem_u32(gD), dchunks, tc::smem_u32(hin),
-                          in_w / 8, in_w, fp16, acc);
+              issue_wgrad(tbase + (l == 0 ? CW0 : (l == 1 ? CW1 : CW2)), del, dchunks, hin, in_w / 8, in_w, fp16, acc);
             started |= 1u << l;
             // data gradient delta_l W_l (W_l's image as an MN-major operand); for l = 0 only the grid columns
             const uint32_t wk = uint32_t(in_w / 8) * 128u;
-            issue_mma_kmajor(tD, tc::smem_u32(gD), dchunks, w_addr + a.layer_off[l], wk, 128u, 2u * wk,
+            issue_mma_kmajor(tD, del, dchunks, w_addr + a.layer_off[l], wk, 128u, 2u * wk,
                              l == 0 ? NGRID : in_w, dwidth / 16, fp16, true);
           }
           tc::mma_commit(&done[i]);
@@ -357,9 +398,8 @@ __global__ void __launch_bounds__(SCAT ? kScatThreadsPerCta : 2 * NWG * kRows + 
           break;
         }
         const uint8_t* gbase = smem + w_region + gg * WG_BYTES;
-        const float* dgs = reinterpret_cast<const float*>(gbase + A_BYTES + 2 * H_BYTES);
-        const float* gp3 = reinterpret_cast<const float*>(gbase + A_BYTES + 3 * H_BYTES + D_BYTES + REC_BYTES) +
-                           (k & 1) * kRows * 4;
+        const float* dgs = reinterpret_cast<const float*>(gbase + Sh::D_OFF);
+        const float* gp3 = reinterpret_cast<const float*>(gbase + Sh::P3_OFF) + (k & 1) * kRows * 4;
         for (int item = sidx; item < kRows * LEVELS; item += kScatThreads) {
           const int r = item % kRows, lv = item / kRows;
           const long q = long(tile) * kRows + r;
@@ -388,6 +428,8 @@ __global__ void __launch_bounds__(SCAT ? kScatThreadsPerCta : 2 * NWG * kRows + 
     const bool sel_on = a.selection != 0;
     const uint32_t tD = tbase + g * DCOLS;
     const uint32_t lane_addr = (uint32_t((warp & 3) * 32) << 16);
+    // this half row's packed words of the parked layers
+    const uint32_t park_addr = tbase + lane_addr + Sh::CPK + uint32_t(g * PARK * (kWidth / 2) + h * (kWidth / 4));
     for (int tile = blockIdx.x * NWG + g; tile < ntiles; tile += gridDim.x * NWG) {
       const int kt = (tile - (blockIdx.x * NWG + g)) / (gridDim.x * NWG);  // this pipeline's tile number
       const long q = long(tile) * kRows + t;
@@ -433,13 +475,12 @@ __global__ void __launch_bounds__(SCAT ? kScatThreadsPerCta : 2 * NWG * kRows + 
         if (l < NL - 1) {
           float v[kWidth / 2];
           tc::tmem_load<kWidth / 32>(tD + lane_addr + uint32_t(h * (kWidth / 2)), v);
-          uint8_t* H = Hs + l * H_BYTES;
-          bool free_h = true;
-          if (SCAT && l == 2 && kt > 0)  // the scatter warps still read the previous tile's gradient here
-            free_h = tc::mbar_wait(&sempty[g], uint32_t(kt - 1) & 1u);
+          uint32_t pk[16];
 #pragma unroll
-          for (int c = 0; c < HC; ++c) store_chunk_relu(H, t, h * HC + c, kWidth / 8, v + 8 * c, fp16);
-          ok = signal_ready(g, leader, &ready[g], fin && free_h && ok);
+          for (int i = 0; i < 16; ++i) pk[i] = tc::pack2_relu(v[2 * i], v[2 * i + 1], fp16);
+          store_half_row(A0 + Sh::fwd_off(l), t, h, pk);
+          if (l < PARK) tc::tmem_store16(park_addr + uint32_t(l * (kWidth / 2)), pk);
+          ok = signal_ready(g, leader, &ready[g], fin && ok);
           if (!ok) break;
         } else {
           tc::tmem_load<K / 8>(tD + lane_addr + uint32_t(h * 2 * K), rh);
@@ -486,6 +527,8 @@ __global__ void __launch_bounds__(SCAT ? kScatThreadsPerCta : 2 * NWG * kRows + 
                                : half_loss_grad<KH, true, false>(hl, mine.x + other.x, mine.y + other.y, 0.f, rr,
                                                                  scale, a.mix, gh, &gsel);
         if (valid && h == 0) loss_acc += double(l);
+        if (SCAT && kt > 0)  // the scatter warps still read the previous tile's gradient in the delta tile
+          ok = tc::mbar_wait(&sempty[g], uint32_t(kt - 1) & 1u) && ok;
         // delta columns: half 0 its lobes' [0, 2K); half 1 its lobes' [2K, 4K),
         // the selection logit's gradient (column 4K) and zero padding to nout
         if (h == 0) {
@@ -522,14 +565,19 @@ __global__ void __launch_bounds__(SCAT ? kScatThreadsPerCta : 2 * NWG * kRows + 
         tc::fence_after_sync();
         float v[kWidth / 2];
         tc::tmem_load<kWidth / 32>(tD + lane_addr + uint32_t(h * (kWidth / 2)), v);
-        const uint8_t* H = Hs + (l - 1) * H_BYTES;
+        uint8_t* H = A0 + Sh::bwd_off(l - 1);  // h_{l-1}, which delta_{l-1} replaces in place
 #pragma unroll
         for (int c = 0; c < HC; ++c) {
           float hv[8], fv[8];
           load_chunk(H, t, h * HC + c, kWidth / 8, hv, fp16);
 #pragma unroll
           for (int i = 0; i < 8; ++i) fv[i] = hv[i] > 0.f ? v[8 * c + i] : 0.f;
-          store_chunk(Dt, t, h * HC + c, kWidth / 8, fv, fp16);
+          store_chunk(H, t, h * HC + c, kWidth / 8, fv, fp16);
+        }
+        if (l >= 2 && l - 2 < PARK) {  // h_{l-2} back from TMEM, over delta_l, whose MMAs are done
+          uint32_t pk[16];
+          tc::tmem_load16(park_addr + uint32_t((l - 2) * (kWidth / 2)), pk);
+          store_half_row(A0 + Sh::bwd_off(l - 2), t, h, pk);
         }
         ok = signal_ready(g, leader, &ready[g], fin && ok);
         if (!ok) break;
@@ -545,9 +593,8 @@ __global__ void __launch_bounds__(SCAT ? kScatThreadsPerCta : 2 * NWG * kRows + 
         ok = bar_red_and(1 + g, 2 * kRows, fin && ok);
         if (!ok) break;
         if constexpr (SCAT) {
-          // hand the gradient to the scatter warps through the third hidden tile
-          float* dgs = reinterpret_cast<float*>(Hs + 2 * H_BYTES);
-          static_assert(NGRID * kRows * 4 <= H_BYTES, "grid gradient staging fits a hidden tile");
+          // hand the gradient to the scatter warps through the delta tile
+          float* dgs = reinterpret_cast<float*>(Dt);
 #pragma unroll
           for (int ch = 0; ch < GCH; ++ch)
             if ((ch & 1) == h) {
@@ -563,7 +610,6 @@ __global__ void __launch_bounds__(SCAT ? kScatThreadsPerCta : 2 * NWG * kRows + 
         // so the level loop below can index it: [feature][row] floats; each
         // half stages and scatters the levels of its own chunks.
         float* dgs = reinterpret_cast<float*>(Dt);
-        static_assert(NGRID * kRows * 4 <= D_BYTES, "grid gradient staging fits the delta tile");
 #pragma unroll
         for (int ch = 0; ch < GCH; ++ch)
           if ((ch & 1) == h) {
@@ -657,9 +703,6 @@ __global__ void __launch_bounds__(SCAT ? kScatThreadsPerCta : 2 * NWG * kRows + 
 template <int F, int LEVELS, int MODE, int SHDEG, int BINS, int K, int NOUTMAX, bool SMOOTH, int NWG, bool SCAT,
           bool REC>
 static nmg_status launch_train(const TrainArgs& a, int grid, cudaStream_t st) {
-  constexpr int NDIR = MODE == 0 ? SHDEG * SHDEG + 3 * BINS : 2 * SHDEG * SHDEG + BINS;
-  constexpr int NENC = (LEVELS * F + NDIR + 15) / 16 * 16;
-  constexpr int DW = NOUTMAX > kWidth ? NOUTMAX : kWidth;
   auto kern = k_fused_train<F, LEVELS, MODE, SHDEG, BINS, K, NOUTMAX, SMOOTH, NWG, SCAT, REC>;
   if constexpr (SCAT) {
     // the register split assumes the kernel was compiled to exactly its launch registers
@@ -673,11 +716,7 @@ static nmg_status launch_train(const TrainArgs& a, int grid, cudaStream_t st) {
     }
     if (regs_ok < 0) return launch_train<F, LEVELS, MODE, SHDEG, BINS, K, NOUTMAX, SMOOTH, NWG, false, REC>(a, grid, st);
   }
-  const size_t smem = size_t((a.f.w_bytes + 1023u) & ~1023u) +
-                      NWG * (size_t(kRows) * NENC * 2 + 3 * size_t(kRows) * kWidth * 2 + size_t(kRows) * DW * 2 +
-                             (REC ? size_t(kRows) * 8 * 4 : 0) + (SCAT ? 2 * size_t(kRows) * 4 * 4 : 0) +
-                             2 * size_t(kRows) * 2 * 4) +
-                      256;
+  const size_t smem = TrainShape<F, LEVELS, MODE, SHDEG, BINS, NOUTMAX, NWG, SCAT, REC>::smem_bytes(a.f.w_bytes);
   nmg_status s = ensure_smem(reinterpret_cast<const void*>(kern), smem);
   if (s != NMG_OK) return s;
   kern<<<grid, SCAT ? kScatThreadsPerCta : 2 * NWG * kRows + 32, smem, st>>>(a);
