@@ -134,44 +134,34 @@ NMG_D bool signal_ready(int g, bool leader, uint64_t* ready, bool ok) {
 }
 
 // Adds one record's grid-feature gradient df[F] of level lv into the table
-// gradient gt with the corner weights of position p3 (grid.h:387-510).
+// gradient gt with the corner weights of position p3 (grid.h:387-510): the
+// four corners at x + xb. Neighbouring lanes take xb = 0 and 1 of the same
+// record: the two corners' entries are adjacent in a dense level, and in the
+// same 16-entry block 15 times in 16 in a hashed one (the x term of the hash
+// is x itself), so each reduction instruction sends a pair's two corners to
+// L2 as one request. 2^18 records: see k_fused_train.
 template <int F, bool SMOOTH>
-NMG_D void scatter_level(const FusedArgs& a, float* gt, int lv, const float (&p3)[3], const float (&df)[F]) {
+NMG_D void scatter_level(const FusedArgs& a, float* gt, int lv, const float (&p3)[3], const float (&df)[F],
+                         uint32_t xb) {
   float w[3];
   uint32_t gc[3];
 #pragma unroll
   for (int d = 0; d < 3; ++d) pos_fract(p3[d], a.enc.scale[lv], SMOOTH ? 1 : 0, &w[d], &gc[d]);
-  const float wxy[4] = {(1.f - w[0]) * (1.f - w[1]), w[0] * (1.f - w[1]), (1.f - w[0]) * w[1], w[0] * w[1]};
+  const float wx = xb ? w[0] : 1.f - w[0];
+  const float wxy[2] = {wx * (1.f - w[1]), wx * w[1]};
   const float wz[2] = {1.f - w[2], w[2]};
-  if constexpr (F == 2) {
-    // Corners x and x+1 of a (y, z) pair often land on adjacent entries (always for dense
-    // levels, for even x on hashed ones: the x term of the hash is x itself); one 16-byte
-    // vector reduction then updates both, halving those atomics' L2 requests.
+  float* lvl = gt + size_t(a.enc.offset[lv]) * F;
 #pragma unroll
-    for (int c = 0; c < 8; c += 2) {
-      const uint32_t yy = gc[1] + ((c >> 1) & 1), zz = gc[2] + (c >> 2);
-      const uint32_t e0 = a.enc.offset[lv] + level_index(a, lv, gc[0], yy, zz);
-      const uint32_t e1 = a.enc.offset[lv] + level_index(a, lv, gc[0] + 1u, yy, zz);
-      const float wt0 = wxy[c & 3] * wz[c >> 2], wt1 = wxy[(c + 1) & 3] * wz[c >> 2];
-      const float2 g0 = make_float2(wt0 * df[0], wt0 * df[1]), g1 = make_float2(wt1 * df[0], wt1 * df[1]);
-      if ((e0 ^ e1) == 1u) {  // entries 2m and 2m+1: one aligned 16-byte pair
-        const bool lo0 = e0 < e1;
-        atomicAdd(reinterpret_cast<float4*>(gt + size_t(lo0 ? e0 : e1) * 2),
-                  lo0 ? make_float4(g0.x, g0.y, g1.x, g1.y) : make_float4(g1.x, g1.y, g0.x, g0.y));
-      } else {
-        atomicAdd(reinterpret_cast<float2*>(gt + size_t(e0) * 2), g0);
-        atomicAdd(reinterpret_cast<float2*>(gt + size_t(e1) * 2), g1);
-      }
-    }
-  } else {
+  for (int c = 0; c < 4; ++c) {
+    const float wt = wxy[c & 1] * wz[c >> 1];
+    const uint32_t e = level_index(a, lv, gc[0] + xb, gc[1] + (c & 1), gc[2] + (c >> 1));
+    if constexpr (F == 2) {
+      atomicAdd(reinterpret_cast<float2*>(lvl + size_t(e) * 2), make_float2(wt * df[0], wt * df[1]));
+    } else {
 #pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      const float wt = wxy[c & 3] * wz[c >> 2];
-      const uint32_t e = a.enc.offset[lv] +
-                         level_index(a, lv, gc[0] + (c & 1), gc[1] + ((c >> 1) & 1), gc[2] + ((c >> 2) & 1));
-#pragma unroll
-      for (int k = 0; k < F; k += 2)
-        atomicAdd(reinterpret_cast<float2*>(gt + size_t(e) * F + k), make_float2(wt * df[k], wt * df[k + 1]));
+      for (int k = 0; k < F; k += 4)
+        atomicAdd(reinterpret_cast<float4*>(lvl + size_t(e) * F + k),
+                  make_float4(wt * df[k], wt * df[k + 1], wt * df[k + 2], wt * df[k + 3]));
     }
   }
 }
@@ -383,8 +373,10 @@ __global__ void __launch_bounds__(SCAT ? kScatThreadsPerCta : 2 * NWG * kRows + 
     // ------------------------------------------------------- scatter warps
     tc::reg_dealloc<kScatRegScatter>();
     // Tiles in the order the compute groups finish them (k-th tile of group
-    // 0, then of group 1, ...); items (level, row) with rows fastest, so a
-    // warp reads consecutive rows of the staged [feature][row] gradient.
+    // 0, then of group 1, ...); items (level, row, x corner) with the x corner
+    // fastest, so a warp reads consecutive rows of the staged [feature][row]
+    // gradient and a pair of lanes shares a row.
+    static_assert(kScatThreads % 2 == 0, "a row's two lanes stay neighbours");
     const int sidx = int(threadIdx.x) - (NWG * 8 + 1) * 32;
     float* gt = ta.grad + ta.n_mlp;
     for (int k = 0; ok; ++k) {
@@ -400,15 +392,15 @@ __global__ void __launch_bounds__(SCAT ? kScatThreadsPerCta : 2 * NWG * kRows + 
         const uint8_t* gbase = smem + w_region + gg * WG_BYTES;
         const float* dgs = reinterpret_cast<const float*>(gbase + Sh::D_OFF);
         const float* gp3 = reinterpret_cast<const float*>(gbase + Sh::P3_OFF) + (k & 1) * kRows * 4;
-        for (int item = sidx; item < kRows * LEVELS; item += kScatThreads) {
-          const int r = item % kRows, lv = item / kRows;
+        for (int item = sidx; item < 2 * kRows * LEVELS; item += kScatThreads) {
+          const int r = (item >> 1) % kRows, lv = item / (2 * kRows);
           const long q = long(tile) * kRows + r;
           if (q < n) {
             const float p3[3] = {gp3[4 * r], gp3[4 * r + 1], gp3[4 * r + 2]};
             float df[F];
 #pragma unroll
             for (int kk = 0; kk < F; ++kk) df[kk] = dgs[(F * lv + kk) * kRows + r];
-            scatter_level<F, SMOOTH>(a, gt, lv, p3, df);
+            scatter_level<F, SMOOTH>(a, gt, lv, p3, df, uint32_t(item & 1));
           }
         }
         tc::mbar_arrive(&sempty[gg]);
@@ -627,7 +619,8 @@ __global__ void __launch_bounds__(SCAT ? kScatThreadsPerCta : 2 * NWG * kRows + 
               float df[F];
 #pragma unroll
               for (int k = 0; k < F; ++k) df[k] = dgs[(F * lv + k) * kRows + t];
-              scatter_level<F, SMOOTH>(a, gt, lv, p3, df);
+              scatter_level<F, SMOOTH>(a, gt, lv, p3, df, 0u);
+              scatter_level<F, SMOOTH>(a, gt, lv, p3, df, 1u);
             }
           }
         }
