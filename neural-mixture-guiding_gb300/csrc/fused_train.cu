@@ -68,23 +68,39 @@ struct TrainArgs {
   nmg_radiance_records rr;
 };
 
-NMG_D void issue_mma_kmajor(uint32_t tmem, uint32_t a_addr, int a_chunks, uint32_t b_addr, uint32_t b_lbo,
-                            uint32_t b_sbo, uint32_t b_step, int N, int ksteps, bool fp16, bool b_mn) {
-  const uint32_t idesc = tc::idesc_f16(kRows, N, fp16, false, b_mn);
-  for (int kk = 0; kk < ksteps; ++kk)
-    tc::mma_f16(tmem, tc::smem_desc(a_addr + kk * 256u, 128u, uint32_t(a_chunks) * 128u),
-                tc::smem_desc(b_addr + kk * b_step, b_lbo, b_sbo), idesc, kk > 0 ? 1u : 0u);
+// D[tmem] (+)= sum over STEPS 16-deep slices of A and B whose descriptors
+// advance by a_step / b_step bytes per slice. The descriptors are formed once
+// and stepped by adding to their address field: one thread issues all of the
+// CTA's MMAs, and building two descriptors per MMA cost it more than the MMAs
+// take.
+template <int STEPS>
+NMG_D void issue_steps(uint32_t tmem, uint64_t a, uint32_t a_step, uint64_t b, uint32_t b_step, uint32_t idesc,
+                       bool accumulate) {
+#pragma unroll
+  for (int kk = 0; kk < STEPS; ++kk)
+    tc::mma_f16(tmem, a + uint64_t(kk * (a_step >> 4)), b + uint64_t(kk * (b_step >> 4)), idesc,
+                (accumulate || kk > 0) ? 1u : 0u);
+}
+
+// A K-major tile (a_chunks chunks a row) times a weight image: forward
+// (b_mn = false, the image K-major, kin / 16 slices) or data gradient (the
+// image of `in_chunks` chunks a row read MN-major).
+template <int STEPS>
+NMG_D void issue_rows(uint32_t tmem, uint32_t a_addr, int a_chunks, uint32_t b_addr, int b_chunks, int N, bool fp16,
+                      bool b_mn) {
+  const uint32_t idesc = tc::idesc_f16(kRows, N, fp16, false, b_mn), bc = uint32_t(b_chunks) * 128u;
+  const uint64_t a = tc::smem_desc(a_addr, 128u, uint32_t(a_chunks) * 128u);
+  const uint64_t b = b_mn ? tc::smem_desc(b_addr, bc, 128u) : tc::smem_desc(b_addr, 128u, bc);
+  issue_steps<STEPS>(tmem, a, 256u, b, b_mn ? 2u * bc : 256u, idesc, false);
 }
 
 // dW (M = 64 rows of `a_tile` chunks, N = columns of `b_tile` chunks) +=
 // a_tile^T b_tile over the 128 rows (K) of both tiles, MN-major views.
 NMG_D void issue_wgrad(uint32_t tmem, uint32_t a_addr, int a_chunks, uint32_t b_addr, int b_chunks, int N,
                        bool fp16, bool accumulate) {
-  const uint32_t idesc = tc::idesc_f16(64, N, fp16, true, true);
-  for (int kk = 0; kk < kRows / 16; ++kk)
-    tc::mma_f16(tmem, tc::smem_desc(a_addr + kk * 2u * a_chunks * 128u, uint32_t(a_chunks) * 128u, 128u),
-                tc::smem_desc(b_addr + kk * 2u * b_chunks * 128u, uint32_t(b_chunks) * 128u, 128u), idesc,
-                (accumulate || kk > 0) ? 1u : 0u);
+  const uint32_t ac = uint32_t(a_chunks) * 128u, bc = uint32_t(b_chunks) * 128u;
+  issue_steps<kRows / 16>(tmem, tc::smem_desc(a_addr, ac, 128u), 2u * ac, tc::smem_desc(b_addr, bc, 128u), 2u * bc,
+                          tc::idesc_f16(64, N, fp16, true, true), accumulate);
 }
 
 // Reads 16-bit row `row` of a core-matrix tile (chunk c) as 8 floats.
@@ -332,30 +348,34 @@ __global__ void __launch_bounds__(SCAT ? kScatThreadsPerCta : 2 * NWG * kRows + 
           last = clock64();
           tc::fence_after_sync();
           uint8_t* gA0 = smem + w_region + i * WG_BYTES;
-          const uint32_t g_addr = tc::smem_u32(gA0);
+          const uint32_t g_addr = tc::smem_u32(gA0), a0_addr = g_addr;
           const uint32_t tD = tbase + i * DCOLS;
           const int s = step[i];
-          if (s < NL) {  // forward layer s
-            const int kin = s == 0 ? NENC : kWidth;
-            const uint32_t a_addr = s == 0 ? g_addr : g_addr + Sh::fwd_off(s - 1);
-            issue_mma_kmajor(tD, a_addr, kin / 8, w_addr + a.layer_off[s], 128u, uint32_t(kin / 8) * 128u, 256u,
-                             s == NL - 1 ? nout : kWidth, kin / 16, fp16, false);
-          } else {  // backward layer l: weight gradient then data gradient
+          if (s == 0) {  // forward layers
+            issue_rows<NENC / 16>(tD, a0_addr, NENC / 8, w_addr + a.layer_off[0], NENC / 8, kWidth, fp16, false);
+          } else if (s < NL) {
+            issue_rows<kWidth / 16>(tD, g_addr + Sh::fwd_off(s - 1), kWidth / 8, w_addr + a.layer_off[s], kWidth / 8,
+                                    s == NL - 1 ? nout : kWidth, fp16, false);
+          } else {  // backward layer l: weight gradient, then data gradient delta_l W_l
             const int l = NL - 1 - (s - NL);
-            const int dchunks = l == NL - 1 ? KC3 : kWidth / 8;
-            const int dwidth = l == NL - 1 ? nout : kWidth;
-            const int in_w = l == 0 ? NENC : kWidth;
-            const uint32_t hin = l == 0 ? g_addr : g_addr + Sh::bwd_off(l - 1), del = g_addr + Sh::bwd_off(l);
+            const uint32_t del = g_addr + Sh::bwd_off(l), w_l = w_addr + a.layer_off[l];
+            const uint32_t hin = l == 0 ? a0_addr : g_addr + Sh::bwd_off(l - 1);
             const bool acc = (started >> l) & 1u;
-            if (l == NL - 1)
-              issue_wgrad(tbase + CW3, hin, kWidth / 8, del, dchunks, dwidth, fp16, acc);
-            else
-              issue_wgrad(tbase + (l == 0 ? CW0 : (l == 1 ? CW1 : CW2)), del, dchunks, hin, in_w / 8, in_w, fp16, acc);
             started |= 1u << l;
-            // data gradient delta_l W_l (W_l's image as an MN-major operand); for l = 0 only the grid columns
-            const uint32_t wk = uint32_t(in_w / 8) * 128u;
-            issue_mma_kmajor(tD, del, dchunks, w_addr + a.layer_off[l], wk, 128u, 2u * wk,
-                             l == 0 ? NGRID : in_w, dwidth / 16, fp16, true);
+            if (l == NL - 1) {
+              issue_wgrad(tbase + CW3, hin, kWidth / 8, del, KC3, nout, fp16, acc);
+              const uint32_t wk = uint32_t(kWidth / 8) * 128u;
+              const uint64_t ad = tc::smem_desc(del, 128u, uint32_t(KC3) * 128u), bd = tc::smem_desc(w_l, wk, 128u);
+              const uint32_t idesc = tc::idesc_f16(kRows, kWidth, fp16, false, true);
+              for (int kk = 0; kk < nout / 16; ++kk)
+                tc::mma_f16(tD, ad + uint64_t(kk * 16), bd + uint64_t(kk * (2u * wk >> 4)), idesc, kk > 0 ? 1u : 0u);
+            } else if (l > 0) {
+              issue_wgrad(tbase + (l == 1 ? CW1 : CW2), del, kWidth / 8, hin, kWidth / 8, kWidth, fp16, acc);
+              issue_rows<kWidth / 16>(tD, del, kWidth / 8, w_l, kWidth / 8, kWidth, fp16, true);
+            } else {  // only the grid columns have parameters below
+              issue_wgrad(tbase + CW0, del, kWidth / 8, hin, NENC / 8, NENC, fp16, acc);
+              issue_rows<kWidth / 16>(tD, del, kWidth / 8, w_l, NENC / 8, NGRID, fp16, true);
+            }
           }
           tc::mma_commit(&done[i]);
           step[i] = (s + 1) % (2 * NL);
