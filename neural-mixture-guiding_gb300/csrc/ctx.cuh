@@ -13,6 +13,7 @@ namespace nmg {
 
 constexpr int kWidth = 64;       // MLP width (the only one compiled)
 constexpr int kMaxLayers = 8;    // weight matrices
+constexpr int kPlainRows = 64;   // rows per tile of the plain network kernels
 
 struct Layout {
   int K, n_out, n_out_pad, n_layers;  // n_layers = hidden_layers + 1 weight matrices
@@ -26,11 +27,12 @@ struct Workspace {
   int cap_q = 0, cap_b = 0;
   // plain path
   float* x = nullptr;      // [cap][n_input]
-  float* enc = nullptr;    // [cap][n_enc_pad]
-  float* h[kMaxLayers] = {};  // [cap][64] activations after ReLU
+  // kept for the plain backward pass, in tiles of [column][kPlainRows rows]
+  float* enc = nullptr;    // n_enc_pad columns
+  float* h[kMaxLayers] = {};  // 64 columns: activations after ReLU
+  float* delta[kMaxLayers] = {};  // each layer's output columns: dL/d(output before ReLU)
   float* raw = nullptr;    // [cap][n_out_pad]
   float* draw = nullptr;   // [cap_b][n_out_pad]
-  float* dh[2] = {};       // [cap_b][max(64, n_enc_pad)] ping-pong deltas
   double* partials = nullptr;  // block partial sums (loss, grad norm)
   int n_partials = 0;
   int* batch_counts = nullptr; // [kMaxFrameBatches] record counts of nmg_train_frame's batches
@@ -69,11 +71,15 @@ struct nmg_ctx {
 
 namespace nmg {
 
+// plain_net.cu
+nmg_status plain_forward(nmg_ctx* c, const nmg_shading* in, const float* x, const int* d_count, int n_max,
+                         const float* weights, bool keep_hidden, float* raw_out, cudaStream_t st);
+nmg_status plain_backward(nmg_ctx* c, const float* x, const int* d_count, int n_max, const float* weights,
+                          float* dparams, cudaStream_t st);
+
 // plain.cu
 nmg_status plain_featurize(nmg_ctx* c, const nmg_shading* in, const int* d_count, int n_max, float* x,
                            cudaStream_t st);
-nmg_status plain_forward(nmg_ctx* c, const float* x, const int* d_count, int n_max, const float* weights,
-                         bool keep_hidden, float* raw_out, cudaStream_t st);
 nmg_status plain_query(nmg_ctx* c, const nmg_shading* in, const float* u4, const int* d_count, int n_max,
                        const nmg_query_out* out, cudaStream_t st);
 nmg_status plain_pdf(nmg_ctx* c, const nmg_shading* in, const float* wi, const int* d_count, int n_max,

@@ -142,8 +142,7 @@ static void free_workspace(nmg_ctx* c) {
   for (auto& h : w.h) cudaFree(h);
   cudaFree(w.raw);
   cudaFree(w.draw);
-  cudaFree(w.dh[0]);
-  cudaFree(w.dh[1]);
+  for (auto& d : w.delta) cudaFree(d);
   cudaFree(w.partials);
   cudaFree(w.batch_counts);
   cudaFree(w.recs);
@@ -176,15 +175,13 @@ static nmg_status reserve(nmg_ctx* c, int max_q, int max_b) {
   A(w.raw, capz * L.n_out_pad);
   w.n_partials = 2 * 2048;
   if (fp32) {
-    A(w.enc, capz * c->enc.n_enc_pad);
-    for (int l = 0; l < L.n_layers - 1; ++l)
-      if (l < 2 || max_b > 0) A(w.h[l], capz * kWidth);
     if (max_b > 0) {
-      const size_t wd = size_t(c->enc.n_enc_pad > kWidth ? c->enc.n_enc_pad : kWidth);
+      const size_t rows = (size_t(max_b) + kPlainRows - 1) / kPlainRows * kPlainRows;
+      A(w.enc, rows * c->enc.n_enc_pad);
+      for (int l = 0; l < L.n_layers - 1; ++l) A(w.h[l], rows * kWidth);
+      for (int l = 0; l < L.n_layers; ++l) A(w.delta[l], rows * L.out[l]);
       A(w.draw, size_t(max_b) * L.n_out_pad);
       A(w.recs, size_t(max_b) * 8);
-      A(w.dh[0], size_t(max_b) * wd);
-      A(w.dh[1], size_t(max_b) * wd);
     }
   }
 #undef A
@@ -414,7 +411,7 @@ nmg_status nmg_infer_raw(nmg_ctx* c, const float* x, int n, int which, float* ra
   nmg_status s = need(c, n, false);
   if (s != NMG_OK || n == 0) return s;
   cudaStream_t st = (cudaStream_t)stream;
-  if (c->cfg.path == NMG_PATH_FP32) return plain_forward(c, x, nullptr, n, which ? c->w_inf : c->w, false, raw, st);
+  if (c->cfg.path == NMG_PATH_FP32) return plain_forward(c, nullptr, x, nullptr, n, which ? c->w_inf : c->w, false, raw, st);
   return fused_infer_raw(c, x, nullptr, n, which, raw, st);
 }
 

@@ -1,0 +1,654 @@
+// plain_net.cu -- the plain FP32 network: encoding, MLP forward, backward
+// through the MLP and the grid, weight gradients.
+//
+// FP32 FMAs on the CUDA cores, every sum in the order of one input after
+// another. What bounds it is those FMAs (13,312 a row for the reference
+// network, 16,384 for the hash-grid one: 72 TFLOP/s measured for plain FMAs on
+// this GPU), so nothing else may be in the way: one kernel per direction keeps
+// a tile of 64 rows in shared memory from the first layer to the last, next to
+// all of the weights. Two blocks of 256 threads per SM, so that one's table
+// gathers run under the other's FMAs. 524,288 queries of the reference network
+// took 1,319 us with one kernel per operation (encoding 377 us, four layers
+// 850 us, all through HBM).
+//
+// For the backward pass the forward kernel leaves the encoded rows and the
+// hidden activations in global memory as tiles of [column][64 rows], the order
+// they have in shared memory; the backward kernel does the same with the
+// deltas, and the weight-gradient kernel reads both.
+#include <string.h>
+
+#include "api_common.cuh"
+#include "ctx.cuh"
+
+namespace nmg {
+
+constexpr int kPlainThreads = 256;
+
+struct PlainNet {
+  EncodingParams enc;
+  int n_layers, n_grid;           // n_grid = levels * feats
+  int in[kMaxLayers], out[kMaxLayers];
+  const float* w[kMaxLayers];     // row-major [out][in]
+  const float* table;
+  uint32_t T[kMaxLevels], sy[kMaxLevels], sz[kMaxLevels];  // entries; dense strides of y and z
+  uint32_t hashed;                // bit l: level l is hashed
+  uint32_t pow2;                  // bit l: T is a power of two
+  const int* d_count;
+  int n_max;
+};
+
+struct PlainFwd {
+  PlainNet net;
+  nmg_shading in;                 // pos non-NULL: featurise these
+  const float* x;                 // else network input rows
+  float* enc_t;                   // NULL, or the tiles kept for the backward pass
+  float* h_t[kMaxLayers];
+  float* raw;                     // [n][ld_raw]
+  int ld_raw;
+  int raw_wide;                   // raw is 16-byte aligned
+};
+
+struct PlainBwd {
+  PlainNet net;
+  const float* x;                 // network input rows
+  const float* draw;              // [n][out of the last layer]
+  const float* h_t[kMaxLayers];
+  float* d_t[kMaxLayers];         // delta tiles of every layer
+  float* gtable;
+  int wide;                       // gtable is 16-byte aligned
+};
+
+NMG_D int plain_count(const PlainNet& p) {
+  if (!p.d_count) return p.n_max;
+  const int n = *p.d_count;
+  return n < 0 ? 0 : (n > p.n_max ? p.n_max : n);
+}
+
+// grid_index with the level's strides and hashing worked out on the host.
+NMG_D uint32_t plain_index(const PlainNet& p, int l, uint32_t x, uint32_t y, uint32_t z) {
+  const uint32_t T = p.T[l];
+  const uint32_t i = (p.hashed >> l) & 1u ? x ^ (y * 2654435761u) ^ (z * 805459861u)
+                                          : x + y * p.sy[l] + z * p.sz[l];
+  if ((p.pow2 >> l) & 1u) return i & (T - 1u);
+  return i < T ? i : i % T;
+}
+
+template <int F> NMG_D void plain_entry(const float* table, uint32_t e, float (&v)[F]) {
+  if constexpr (F == 1) {
+    v[0] = __ldg(table + e);
+  } else if constexpr (F == 2) {
+    const float2 t = __ldg(reinterpret_cast<const float2*>(table) + e);
+    v[0] = t.x, v[1] = t.y;
+  } else {
+#pragma unroll
+    for (int k = 0; k < F / 4; ++k) {
+      const float4 t = __ldg(reinterpret_cast<const float4*>(table) + size_t(e) * (F / 4) + k);
+      v[4 * k] = t.x, v[4 * k + 1] = t.y, v[4 * k + 2] = t.z, v[4 * k + 3] = t.w;
+    }
+  }
+}
+
+// Part `part` of 4 of the featurisation of one query (featurize<false>'s
+// expressions): position, outgoing direction, normal, roughness.
+NMG_D void featurize_part(const EncodingParams& e, const nmg_shading& in, long q, int part, int r, float* xs) {
+  if (part == 0) {
+    const f3 pos = load3(in.pos, q);
+    const float p[3] = {pos.x, pos.y, pos.z};
+    const float infl = aabb_inflation(e.aabb);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) xs[d * kPlainRows + r] = normalize_coord(e.aabb, infl, d, p[d]);
+  } else if (part == 1) {
+    const f3 w = normalize3(load3(in.wo, q));
+    xs[3 * kPlainRows + r] = (w.x + 1.f) * 0.5f;
+    xs[4 * kPlainRows + r] = (w.y + 1.f) * 0.5f;
+    xs[5 * kPlainRows + r] = (w.z + 1.f) * 0.5f;
+  } else if (part == 2) {
+    const f3 nn = normalize3(load3(in.normal, q));
+    if (e.input_mode == 0) {
+      const float th = acosf(fminf(1.f, fmaxf(-1.f, nn.z)));
+      float ph = atan2f(nn.y, nn.x);
+      if (ph < 0.f) ph += NMG_TWO_PI;
+      xs[6 * kPlainRows + r] = float(double(th) / 3.14159265358979323846);
+      xs[7 * kPlainRows + r] = ph / NMG_TWO_PI;
+    } else {
+      xs[6 * kPlainRows + r] = (nn.x + 1.f) * 0.5f;
+      xs[7 * kPlainRows + r] = (nn.y + 1.f) * 0.5f;
+      xs[8 * kPlainRows + r] = (nn.z + 1.f) * 0.5f;
+    }
+  } else {
+    xs[(e.input_mode == 0 ? 8 : 9) * kPlainRows + r] = 1.f - expf(-in.roughness[q]);
+  }
+}
+
+// Direction columns of row r (encode_directional's), DIR 0: any degree and bin
+// count, by the row's last thread; 1 and 2: the hash-grid (SH 4 twice, 4 bins)
+// and the reference preset (SH 2, three one-blobs of 4 bins), unrolled and
+// split over the row's four threads.
+template <int DIR>
+NMG_D void plain_directional(const EncodingParams& e, const float* xs, float* act, int n_grid, int r, int part) {
+  auto x = [&](int d) { return xs[d * kPlainRows + r]; };
+  if constexpr (DIR == 0) {
+    if (part != 3) return;
+    float xr[10], rest[64];
+    for (int d = 0; d < 10; ++d) xr[d] = d < e.n_input ? x(d) : 0.f;
+    encode_directional(e, xr, rest);
+    for (int k = n_grid; k < e.n_enc_pad; ++k) act[k * kPlainRows + r] = rest[k - n_grid];
+  } else {
+    constexpr int SH = DIR == 1 ? 4 : 2, SH2 = SH * SH;
+    float* o = act + n_grid * kPlainRows + r;
+    if (part == 0 || (DIR == 1 && part == 1)) {
+      const int b = part == 0 ? 3 : 6;
+      float d[16];
+      sh_basis(SH, x(b) * 2.f - 1.f, x(b + 1) * 2.f - 1.f, x(b + 2) * 2.f - 1.f, d);
+#pragma unroll
+      for (int k = 0; k < SH2; ++k) o[(part * SH2 + k) * kPlainRows] = d[k];
+    } else if (DIR == 1 && part == 2) {
+      float d[4];
+      oneblob(4, x(9), d);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) o[(2 * SH2 + k) * kPlainRows] = d[k];
+    } else if (DIR == 1) {
+      for (int k = n_grid + 2 * SH2 + 4; k < e.n_enc_pad; ++k) act[k * kPlainRows + r] = 1.f;
+    } else {
+      float d[4];
+      oneblob(4, x(5 + part), d);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) o[(SH2 + 4 * (part - 1) + k) * kPlainRows] = d[k];
+      if (part == 3)
+        for (int k = n_grid + SH2 + 12; k < e.n_enc_pad; ++k) act[k * kPlainRows + r] = 1.f;
+    }
+  }
+}
+
+// Thread tile of the matrix products: 4 rows x 4 columns. A warp covers 16
+// rows x 32 columns, so that each of its two 16-byte shared loads per step is
+// one wavefront; the block covers 64 x 64 at a time.
+struct PlainTile {
+  int row, col;
+  NMG_D PlainTile() {
+    const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    row = 16 * (wid & 3) + 4 * (lane & 3);
+    col = 32 * (wid >> 2) + 4 * (lane >> 2);
+  }
+};
+
+// acc[column][row] = sum over k < n of A[k][row] B[k][col], k ascending.
+NMG_D void plain_product(const float* A, const float* B, int ldb, int n, float (&acc)[4][4]) {
+#pragma unroll
+  for (int c = 0; c < 4; ++c)
+#pragma unroll
+    for (int r = 0; r < 4; ++r) acc[c][r] = 0.f;
+#pragma unroll 4
+  for (int k = 0; k < n; ++k) {
+    const float4 a = *reinterpret_cast<const float4*>(A + k * kPlainRows);
+    const float4 b = *reinterpret_cast<const float4*>(B + k * ldb);
+    const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+#pragma unroll
+      for (int r = 0; r < 4; ++r) acc[c][r] = fmaf(av[r], bv[c], acc[c][r]);
+  }
+}
+
+constexpr int kPlainPad = 4;  // floats after each transposed weight row: its 16-byte stores spread over the banks
+
+template <int F, int DIR>
+__global__ void __launch_bounds__(kPlainThreads, 2) k_plain_forward(const __grid_constant__ PlainFwd a) {
+  extern __shared__ __align__(16) float sm[];
+  const PlainNet& p = a.net;
+  const int L = p.n_layers, n_enc = p.in[0], n_grid = p.n_grid;
+  float* W = sm;  // per layer [in][out + pad]
+  int w_floats = 0;
+  for (int l = 0; l < L; ++l) {
+    const int nin = p.in[l], nout = p.out[l], ld = nout + kPlainPad, q4 = nin / 4;
+    // 8 output rows x 4 groups of 4 inputs per warp: whole sectors in, two-way conflicts out
+    for (int i = threadIdx.x; i < q4 * nout; i += kPlainThreads) {
+      const int blk = i >> 5, ln = i & 31;
+      const int j = (blk / (q4 / 4)) * 8 + (ln >> 2), k = (blk % (q4 / 4)) * 4 + (ln & 3);
+      const float4 v = __ldg(reinterpret_cast<const float4*>(p.w[l] + size_t(j) * nin) + k);
+      float* d = W + w_floats + 4 * k * ld + j;
+      d[0] = v.x;
+      d[ld] = v.y;
+      d[2 * ld] = v.z;
+      d[3 * ld] = v.w;
+    }
+    w_floats += nin * ld;
+  }
+  float* act = sm + w_floats;                                    // [max(n_enc, 64)][64]
+  float* xs = act + (n_enc > kWidth ? n_enc : kWidth) * kPlainRows;  // [10][64]
+  const int n = plain_count(p);
+  const int r = threadIdx.x % kPlainRows, part = threadIdx.x / kPlainRows;
+  const PlainTile tl;
+  const int tiles = (n + kPlainRows - 1) / kPlainRows;
+  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    const long q0 = long(tile) * kPlainRows, q = q0 + r;
+    __syncthreads();
+    if (a.in.pos) {
+      if (q < n) {
+        featurize_part(p.enc, a.in, q, part, r, xs);
+      } else if (part == 0) {
+        for (int d = 0; d < p.enc.n_input; ++d) xs[d * kPlainRows + r] = 0.f;
+      }
+    } else {
+      const int ni = p.enc.n_input;
+      for (int i = threadIdx.x; i < kPlainRows * ni; i += kPlainThreads) {
+        const int rr = i / ni, d = i - rr * ni;
+        xs[d * kPlainRows + rr] = q0 + rr < n ? a.x[q0 * ni + i] : 0.f;
+      }
+    }
+    __syncthreads();
+    // ---- encoding: the row's four threads take every fourth level each
+    for (int l = part; l < p.enc.levels; l += 4) {
+      float w[3];
+      uint32_t g[3];
+#pragma unroll
+      for (int d = 0; d < 3; ++d) pos_fract(xs[d * kPlainRows + r], p.enc.scale[l], p.enc.smoothstep, &w[d], &g[d]);
+      const float* tab = p.table + size_t(p.enc.offset[l]) * F;
+      float acc[F];
+#pragma unroll
+      for (int f = 0; f < F; ++f) acc[f] = 0.f;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const float wt = ((k & 1 ? w[0] : 1.f - w[0]) * (k & 2 ? w[1] : 1.f - w[1])) * (k & 4 ? w[2] : 1.f - w[2]);
+        float v[F];
+        plain_entry<F>(tab, plain_index(p, l, g[0] + (k & 1), g[1] + ((k >> 1) & 1), g[2] + (k >> 2)), v);
+#pragma unroll
+        for (int f = 0; f < F; ++f) acc[f] = fmaf(wt, v[f], acc[f]);
+      }
+#pragma unroll
+      for (int f = 0; f < F; ++f) act[(l * F + f) * kPlainRows + r] = acc[f];
+    }
+    plain_directional<DIR>(p.enc, xs, act, n_grid, r, part);
+    __syncthreads();
+    if (a.enc_t) {
+      float4* dst = reinterpret_cast<float4*>(a.enc_t + size_t(tile) * kPlainRows * n_enc);
+      for (int i = threadIdx.x; i < n_enc * kPlainRows / 4; i += kPlainThreads)
+        dst[i] = reinterpret_cast<const float4*>(act)[i];
+    }
+    // ---- layers
+    const float* Wl = W;
+    for (int l = 0; l < L; ++l) {
+      const int nin = p.in[l], nout = p.out[l], ld = nout + kPlainPad;
+      float acc[4][4];
+      if (l == L - 1) {
+        for (int c0 = tl.col; c0 < nout; c0 += kWidth) {
+          plain_product(act + tl.row, Wl + c0, ld, nin, acc);
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            if (q0 + tl.row + i < n) {
+              float* dst = a.raw + (q0 + tl.row + i) * a.ld_raw + c0;
+              if (a.raw_wide) {
+                *reinterpret_cast<float4*>(dst) = make_float4(acc[0][i], acc[1][i], acc[2][i], acc[3][i]);
+              } else {
+#pragma unroll
+                for (int c = 0; c < 4; ++c) dst[c] = acc[c][i];
+              }
+            }
+        }
+        break;
+      }
+      plain_product(act + tl.row, Wl + tl.col, ld, nin, acc);  // hidden layers are kWidth wide
+      __syncthreads();
+      float* keep = a.h_t[l] ? a.h_t[l] + size_t(tile) * kPlainRows * kWidth : nullptr;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const float4 v = make_float4(fmaxf(acc[c][0], 0.f), fmaxf(acc[c][1], 0.f), fmaxf(acc[c][2], 0.f),
+                                     fmaxf(acc[c][3], 0.f));
+        const int at = (tl.col + c) * kPlainRows + tl.row;
+        *reinterpret_cast<float4*>(act + at) = v;
+        if (keep) *reinterpret_cast<float4*>(keep + at) = v;
+      }
+      __syncthreads();
+      Wl += nin * ld;
+    }
+  }
+}
+
+// Adds one record's grid-feature gradient g[F] at corner x + xb of level l's
+// four (y, z) into the table gradient (grid.h:387-510). Neighbouring lanes
+// take the two x corners of a record, which mostly share a 128-byte line: one
+// L2 request for both.
+template <int F>
+NMG_D void plain_scatter(const PlainNet& p, int l, const float (&pos)[3], const float (&g)[F], uint32_t xb,
+                         float* gtable, bool wide) {
+  float w[3];
+  uint32_t gc[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) pos_fract(pos[d], p.enc.scale[l], p.enc.smoothstep, &w[d], &gc[d]);
+  const float wx = xb ? w[0] : 1.f - w[0];
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    const float wt = (wx * (c & 1 ? w[1] : 1.f - w[1])) * (c & 2 ? w[2] : 1.f - w[2]);
+    const uint32_t e = p.enc.offset[l] + plain_index(p, l, gc[0] + xb, gc[1] + (c & 1), gc[2] + (c >> 1));
+    float* dst = gtable + size_t(e) * F;
+    if (F == 1 || !wide) {
+#pragma unroll
+      for (int k = 0; k < F; ++k) atomicAdd(dst + k, wt * g[k]);
+    } else if constexpr (F == 2) {
+      atomicAdd(reinterpret_cast<float2*>(dst), make_float2(wt * g[0], wt * g[1]));
+    } else {
+#pragma unroll
+      for (int k = 0; k + 3 < F; k += 4)
+        atomicAdd(reinterpret_cast<float4*>(dst + k),
+                  make_float4(wt * g[k], wt * g[k + 1], wt * g[k + 2], wt * g[k + 3]));
+    }
+  }
+}
+
+// Deltas of every layer from dL/draw, and the grid gradient. Of layer 0's
+// input only the grid columns have parameters below.
+template <int F>
+__global__ void __launch_bounds__(kPlainThreads, 2) k_plain_backward(const __grid_constant__ PlainBwd a) {
+  extern __shared__ __align__(16) float sm[];
+  const PlainNet& p = a.net;
+  const int L = p.n_layers, nout = p.out[L - 1], g4 = (p.n_grid + 3) / 4 * 4;
+  float* W = sm;  // per layer, the last first: [out][in], layer 0: [out][g4]
+  int w_floats = 0;
+  for (int l = L - 1; l >= 0; --l) {
+    const int ld = l == 0 ? g4 : p.in[l];
+    for (int i = threadIdx.x; i < p.out[l] * (ld / 4); i += kPlainThreads) {
+      const int j = i / (ld / 4), k = i - j * (ld / 4);
+      reinterpret_cast<float4*>(W + w_floats)[i] = __ldg(reinterpret_cast<const float4*>(p.w[l] + size_t(j) * p.in[l]) + k);
+    }
+    w_floats += p.out[l] * ld;
+  }
+  int dw = nout > kWidth ? nout : kWidth;
+  if (g4 > dw) dw = g4;
+  float* D = sm + w_floats;          // [dw][64]
+  float* xs = D + dw * kPlainRows;   // [3][64]
+  const int n = plain_count(p), ni = p.enc.n_input;
+  const PlainTile tl;
+  const int tiles = (n + kPlainRows - 1) / kPlainRows;
+  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    const long q0 = long(tile) * kPlainRows;
+    __syncthreads();
+    {
+      float* keep = a.d_t[L - 1] + size_t(tile) * kPlainRows * nout;
+      for (int i = threadIdx.x; i < kPlainRows * (nout / 4); i += kPlainThreads) {
+        const int r = i % kPlainRows, k = i / kPlainRows;
+        const float4 v = q0 + r < n ? __ldg(reinterpret_cast<const float4*>(a.draw + (q0 + r) * nout) + k)
+                                    : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float e[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          D[(4 * k + c) * kPlainRows + r] = e[c];
+          keep[(4 * k + c) * kPlainRows + r] = e[c];
+        }
+      }
+      if (threadIdx.x < 3 * kPlainRows) {
+        const int r = threadIdx.x % kPlainRows, d = threadIdx.x / kPlainRows;
+        xs[threadIdx.x] = q0 + r < n ? a.x[(q0 + r) * ni + d] : 0.f;
+      }
+    }
+    __syncthreads();
+    const float* Wl = W;
+    float acc[4][4];
+    for (int l = L - 1; l >= 1; --l) {
+      const size_t at0 = size_t(tile) * kPlainRows * kWidth;
+      float4 h[4];
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+        h[c] = __ldg(reinterpret_cast<const float4*>(a.h_t[l - 1] + at0 + (tl.col + c) * kPlainRows + tl.row));
+      plain_product(D + tl.row, Wl + tl.col, kWidth, p.out[l], acc);
+      __syncthreads();
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const float4 v = make_float4(h[c].x > 0.f ? acc[c][0] : 0.f, h[c].y > 0.f ? acc[c][1] : 0.f,
+                                     h[c].z > 0.f ? acc[c][2] : 0.f, h[c].w > 0.f ? acc[c][3] : 0.f);
+        const int at = (tl.col + c) * kPlainRows + tl.row;
+        *reinterpret_cast<float4*>(D + at) = v;
+        *reinterpret_cast<float4*>(a.d_t[l - 1] + at0 + at) = v;
+      }
+      __syncthreads();
+      Wl += p.out[l] * kWidth;
+    }
+    // layer 0: at most 128 grid columns, in two rounds of 64
+    float acc2[4][4];
+    const bool c1 = tl.col < g4, c2 = tl.col + kWidth < g4;
+    if (c1) plain_product(D + tl.row, Wl + tl.col, g4, kWidth, acc);
+    if (c2) plain_product(D + tl.row, Wl + tl.col + kWidth, g4, kWidth, acc2);
+    __syncthreads();
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      if (c1)
+        *reinterpret_cast<float4*>(D + (tl.col + c) * kPlainRows + tl.row) =
+            make_float4(acc[c][0], acc[c][1], acc[c][2], acc[c][3]);
+      if (c2)
+        *reinterpret_cast<float4*>(D + (tl.col + kWidth + c) * kPlainRows + tl.row) =
+            make_float4(acc2[c][0], acc2[c][1], acc2[c][2], acc2[c][3]);
+    }
+    __syncthreads();
+    const int r = (threadIdx.x >> 1) % kPlainRows;
+    if (q0 + r < n) {
+      const float pos[3] = {xs[r], xs[kPlainRows + r], xs[2 * kPlainRows + r]};
+      for (int l = threadIdx.x / (2 * kPlainRows); l < p.enc.levels; l += kPlainThreads / (2 * kPlainRows)) {
+        float g[F];
+#pragma unroll
+        for (int f = 0; f < F; ++f) g[f] = D[(l * F + f) * kPlainRows + r];
+        plain_scatter<F>(p, l, pos, g, threadIdx.x & 1u, a.gtable, a.wide != 0);
+      }
+    }
+  }
+}
+
+// dW[j][i] += sum over rows of delta[j][row] input[i][row] for one 64 x 64
+// block of one layer's matrix (blockIdx.y), over this block's share of the
+// tiles. Thread (j, i) = (8 lanes x 2 warps, 4 lanes x 4 warps) holds every
+// 16th row and column: a 16-byte shared load of four rows of a column is then
+// one wavefront (pitch 68 floats).
+struct PlainWgradBlock {
+  const float *d_t, *x_t;  // tiles [nout][64], [nin][64]
+  float* dw;
+  int nout, nin, j0, i0;
+};
+constexpr int kMaxWgradBlocks = 4 * kMaxLayers;
+struct PlainWgrad {
+  PlainWgradBlock blk[kMaxWgradBlocks];
+  const int* d_count;
+  int n_max;
+};
+constexpr int kWgradPitch = kPlainRows + 4;
+
+__global__ void __launch_bounds__(kPlainThreads, 3) k_plain_wgrad(const __grid_constant__ PlainWgrad a) {
+  __shared__ __align__(16) float Ds[64 * kWgradPitch], Xs[64 * kWgradPitch];
+  const PlainWgradBlock& b = a.blk[blockIdx.y];
+  int n = a.n_max;
+  if (a.d_count) n = *a.d_count < 0 ? 0 : (*a.d_count > n ? n : *a.d_count);
+  const int tiles = (n + kPlainRows - 1) / kPlainRows;
+  const int nj = b.nout - b.j0 < 64 ? b.nout - b.j0 : 64, nx = b.nin - b.i0 < 64 ? b.nin - b.i0 : 64;
+  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int i = (lane & 7) + 8 * (wid & 1), j = (lane >> 3) + 4 * (wid >> 1);
+  float acc[4][4] = {};
+  // this thread's four 16-byte pieces of either tile (column c / 16, rows 4 (c % 16) ..)
+  float4 dv[4], xv[4];
+  auto fetch = [&](int tile) {
+    const float* d = b.d_t + (size_t(tile) * b.nout + b.j0) * kPlainRows;
+    const float* x = b.x_t + (size_t(tile) * b.nin + b.i0) * kPlainRows;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int c = threadIdx.x + k * kPlainThreads;
+      const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+      dv[k] = c / 16 < nj ? __ldg(reinterpret_cast<const float4*>(d) + c) : z;
+      xv[k] = c / 16 < nx ? __ldg(reinterpret_cast<const float4*>(x) + c) : z;
+    }
+  };
+  int tile = blockIdx.x;
+  if (tile < tiles) fetch(tile);
+  for (; tile < tiles; tile += gridDim.x) {
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int c = threadIdx.x + k * kPlainThreads;
+      *reinterpret_cast<float4*>(Ds + (c / 16) * kWgradPitch + 4 * (c % 16)) = dv[k];
+      *reinterpret_cast<float4*>(Xs + (c / 16) * kWgradPitch + 4 * (c % 16)) = xv[k];
+    }
+    __syncthreads();
+    if (tile + gridDim.x < tiles) fetch(tile + gridDim.x);
+    if (i < nx && j < nj) {
+#pragma unroll 2
+      for (int r = 0; r < kPlainRows; r += 4) {
+        float4 d[4], x[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          d[k] = *reinterpret_cast<const float4*>(Ds + (j + 16 * k) * kWgradPitch + r);
+          x[k] = *reinterpret_cast<const float4*>(Xs + (i + 16 * k) * kWgradPitch + r);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+          for (int v = 0; v < 4; ++v) {
+            acc[u][v] = fmaf(d[u].x, x[v].x, acc[u][v]);
+            acc[u][v] = fmaf(d[u].y, x[v].y, acc[u][v]);
+            acc[u][v] = fmaf(d[u].z, x[v].z, acc[u][v]);
+            acc[u][v] = fmaf(d[u].w, x[v].w, acc[u][v]);
+          }
+      }
+    }
+  }
+  if (int(blockIdx.x) >= tiles) return;
+#pragma unroll
+  for (int u = 0; u < 4; ++u)
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+      const int jj = j + 16 * u, ii = i + 16 * v;
+      if (jj < nj && ii < nx) atomicAdd(b.dw + size_t(b.j0 + jj) * b.nin + b.i0 + ii, acc[u][v]);
+    }
+}
+
+// ------------------------------------------------------------ host launchers
+static PlainNet plain_net(const nmg_ctx* c, const float* weights, const int* d_count, int n_max) {
+  PlainNet p;
+  memset(&p, 0, sizeof(p));
+  p.enc = c->enc;
+  p.n_layers = c->lay.n_layers;
+  p.n_grid = c->enc.levels * c->enc.feats;
+  for (int l = 0; l < p.n_layers; ++l) {
+    p.in[l] = c->lay.in[l];
+    p.out[l] = c->lay.out[l];
+    p.w[l] = weights + c->lay.off[l];
+  }
+  p.table = weights + c->lay.n_mlp;
+  for (int l = 0; l < c->enc.levels; ++l) {  // grid_index's strides (grid.h:171-187)
+    const uint32_t T = c->enc.offset[l + 1] - c->enc.offset[l];
+    uint32_t s[3] = {0, 0, 0}, stride = 1;
+    for (int d = 0; d < 3; ++d)
+      if (stride <= T) {
+        s[d] = stride;
+        stride *= c->enc.res[l];
+      }
+    p.T[l] = T;
+    p.sy[l] = s[1];
+    p.sz[l] = s[2];
+    if (c->enc.grid_hash && T < stride) p.hashed |= 1u << l;
+    if ((T & (T - 1u)) == 0u) p.pow2 |= 1u << l;
+  }
+  p.d_count = d_count;
+  p.n_max = n_max;
+  return p;
+}
+
+static int plain_grid(int n_max) {
+  const long tiles = (long(n_max) + kPlainRows - 1) / kPlainRows, cap = 2L * sm_count();
+  return int(tiles < 1 ? 1 : (tiles < cap ? tiles : cap));
+}
+
+template <int F, int DIR>
+static nmg_status launch_forward(const PlainFwd& a, size_t smem, cudaStream_t st) {
+  auto kern = k_plain_forward<F, DIR>;
+  NMG_TRY(ensure_smem(reinterpret_cast<const void*>(kern), smem));
+  kern<<<plain_grid(a.net.n_max), kPlainThreads, smem, st>>>(a);
+  return check_launch("k_plain_forward");
+}
+
+// Encode + MLP forward of shading data (in non-NULL) or network input rows x.
+// With keep_hidden the encoded rows and the activations stay in the workspace
+// for the backward pass.
+nmg_status plain_forward(nmg_ctx* c, const nmg_shading* in, const float* x, const int* d_count, int n_max,
+                         const float* weights, bool keep_hidden, float* raw_out, cudaStream_t st) {
+  Workspace& w = c->ws;
+  PlainFwd a;
+  memset(&a, 0, sizeof(a));
+  a.net = plain_net(c, weights, d_count, n_max);
+  if (in) a.in = *in;
+  a.x = x;
+  a.raw = raw_out;
+  a.ld_raw = c->lay.n_out_pad;
+  a.raw_wide = aligned16(raw_out);
+  if (keep_hidden) {
+    a.enc_t = w.enc;
+    for (int l = 0; l < c->lay.n_layers - 1; ++l) a.h_t[l] = w.h[l];
+  }
+  const int ne = c->enc.n_enc_pad;
+  size_t fl = size_t(ne > kWidth ? ne : kWidth) * kPlainRows + 10 * kPlainRows;
+  for (int l = 0; l < c->lay.n_layers; ++l) fl += size_t(c->lay.in[l]) * (c->lay.out[l] + kPlainPad);
+  const size_t smem = fl * sizeof(float);
+  const EncodingParams& e = c->enc;
+  const bool hash = e.input_mode == 1 && e.sh_degree == 4 && e.oneblob_bins == 4;
+  const bool ref = e.input_mode == 0 && e.sh_degree == 2 && e.oneblob_bins == 4;
+  switch (e.feats) {
+    case 1: return launch_forward<1, 0>(a, smem, st);
+    case 2: return hash ? launch_forward<2, 1>(a, smem, st) : launch_forward<2, 0>(a, smem, st);
+    case 4: return ref ? launch_forward<4, 2>(a, smem, st) : launch_forward<4, 0>(a, smem, st);
+    case 8: return launch_forward<8, 0>(a, smem, st);
+  }
+  return set_error(NMG_ERR_UNSUPPORTED, "grid_features=%d", e.feats);
+}
+
+template <int F>
+static nmg_status launch_backward(const PlainBwd& a, size_t smem, cudaStream_t st) {
+  auto kern = k_plain_backward<F>;
+  NMG_TRY(ensure_smem(reinterpret_cast<const void*>(kern), smem));
+  kern<<<plain_grid(a.net.n_max), kPlainThreads, smem, st>>>(a);
+  return check_launch("k_plain_backward");
+}
+
+// Backward through the MLP and the grid from dL/draw held in w.draw, after a
+// forward pass that kept its activations; adds into dparams (layout of the
+// parameters).
+nmg_status plain_backward(nmg_ctx* c, const float* x, const int* d_count, int n_max, const float* weights,
+                          float* dparams, cudaStream_t st) {
+  const Layout& L = c->lay;
+  Workspace& w = c->ws;
+  PlainBwd a;
+  memset(&a, 0, sizeof(a));
+  a.net = plain_net(c, weights, d_count, n_max);
+  a.x = x;
+  a.draw = w.draw;
+  for (int l = 0; l < L.n_layers; ++l) {
+    a.h_t[l] = w.h[l];
+    a.d_t[l] = w.delta[l];
+  }
+  a.gtable = dparams + L.n_mlp;
+  a.wide = aligned16(a.gtable);
+  const int g4 = (a.net.n_grid + 3) / 4 * 4;
+  int dw = L.n_out_pad > kWidth ? L.n_out_pad : kWidth;
+  if (g4 > dw) dw = g4;
+  size_t fl = size_t(dw) * kPlainRows + 3 * kPlainRows + size_t(kWidth) * g4;
+  for (int l = 1; l < L.n_layers; ++l) fl += size_t(L.in[l]) * L.out[l];
+  const size_t smem = fl * sizeof(float);
+  switch (c->enc.feats) {
+    case 1: NMG_TRY(launch_backward<1>(a, smem, st)); break;
+    case 2: NMG_TRY(launch_backward<2>(a, smem, st)); break;
+    case 4: NMG_TRY(launch_backward<4>(a, smem, st)); break;
+    case 8: NMG_TRY(launch_backward<8>(a, smem, st)); break;
+    default: return set_error(NMG_ERR_UNSUPPORTED, "grid_features=%d", c->enc.feats);
+  }
+  PlainWgrad g;
+  memset(&g, 0, sizeof(g));
+  int nb = 0;
+  for (int l = 0; l < L.n_layers; ++l)
+    for (int j0 = 0; j0 < L.out[l]; j0 += 64)
+      for (int i0 = 0; i0 < L.in[l]; i0 += 64)
+        g.blk[nb++] = PlainWgradBlock{w.delta[l], l == 0 ? w.enc : w.h[l - 1], dparams + L.off[l],
+                                      L.out[l], L.in[l], j0, i0};
+  g.d_count = d_count;
+  g.n_max = n_max;
+  // three blocks per SM in all; each adds its 64 x 64 sums once
+  const long tiles = (long(n_max) + kPlainRows - 1) / kPlainRows;
+  long gx = (3L * sm_count() + nb - 1) / nb;
+  if (gx > tiles) gx = tiles;
+  k_plain_wgrad<<<dim3(unsigned(gx < 1 ? 1 : gx), unsigned(nb)), kPlainThreads, 0, st>>>(g);
+  return check_launch("k_plain_wgrad");
+}
+
+}  // namespace nmg
