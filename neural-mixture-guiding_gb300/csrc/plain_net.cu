@@ -6,10 +6,15 @@
 // network, 16,384 for the hash-grid one: 72 TFLOP/s measured for plain FMAs on
 // this GPU), so nothing else may be in the way: one kernel per direction keeps
 // a tile of 64 rows in shared memory from the first layer to the last, next to
-// all of the weights. Two blocks of 256 threads per SM, so that one's table
-// gathers run under the other's FMAs. 524,288 queries of the reference network
-// took 1,319 us with one kernel per operation (encoding 377 us, four layers
-// 850 us, all through HBM).
+// all of the weights. Four warps of a block do the matrix products of one tile
+// while the other four gather the next tile's table entries (forward) or
+// scatter the last tile's grid gradient (backward); two blocks per SM. A
+// product thread holds 4 rows x 8 columns, three 16-byte shared loads per 32
+// FMAs. The forward kernel takes 409 us for the queries above, bound by the
+// products' shared loads (472 us with 4 x 4 per thread on all eight warps and
+// the roles one after the other, the shared-memory pipe 80% busy; 493 us at 2
+// rows x 16 columns, 444 us with eight gathering warps, 430 us on 128-row
+// tiles at 8 x 4).
 //
 // For the backward pass the forward kernel leaves the encoded rows and the
 // hidden activations in global memory as tiles of [column][64 rows], the order
@@ -22,7 +27,8 @@
 
 namespace nmg {
 
-constexpr int kPlainThreads = 256;
+constexpr int kProduct = 128, kMovers = 128;  // threads of a block's two roles, the product warps first
+constexpr int kPlainThreads = kProduct + kMovers;
 
 struct PlainNet {
   EncodingParams enc;
@@ -88,21 +94,21 @@ template <int F> NMG_D void plain_entry(const float* table, uint32_t e, float (&
   }
 }
 
-// Part `part` of 4 of the featurisation of one query (featurize<false>'s
+// Part h of 4 of the featurisation of one query (featurize<false>'s
 // expressions): position, outgoing direction, normal, roughness.
-NMG_D void featurize_part(const EncodingParams& e, const nmg_shading& in, long q, int part, int r, float* xs) {
-  if (part == 0) {
+NMG_D void featurize_part(const EncodingParams& e, const nmg_shading& in, long q, int h, int r, float* xs) {
+  if (h == 0) {
     const f3 pos = load3(in.pos, q);
     const float p[3] = {pos.x, pos.y, pos.z};
     const float infl = aabb_inflation(e.aabb);
 #pragma unroll
     for (int d = 0; d < 3; ++d) xs[d * kPlainRows + r] = normalize_coord(e.aabb, infl, d, p[d]);
-  } else if (part == 1) {
+  } else if (h == 1) {
     const f3 w = normalize3(load3(in.wo, q));
     xs[3 * kPlainRows + r] = (w.x + 1.f) * 0.5f;
     xs[4 * kPlainRows + r] = (w.y + 1.f) * 0.5f;
     xs[5 * kPlainRows + r] = (w.z + 1.f) * 0.5f;
-  } else if (part == 2) {
+  } else if (h == 2) {
     const f3 nn = normalize3(load3(in.normal, q));
     if (e.input_mode == 0) {
       const float th = acosf(fminf(1.f, fmaxf(-1.f, nn.z)));
@@ -121,14 +127,13 @@ NMG_D void featurize_part(const EncodingParams& e, const nmg_shading& in, long q
 }
 
 // Direction columns of row r (encode_directional's), DIR 0: any degree and bin
-// count, by the row's last thread; 1 and 2: the hash-grid (SH 4 twice, 4 bins)
-// and the reference preset (SH 2, three one-blobs of 4 bins), unrolled and
-// split over the row's four threads.
+// count, as part 3; 1 and 2: the hash-grid (SH 4 twice, 4 bins) and the
+// reference preset (SH 2, three one-blobs of 4 bins), unrolled, in four parts.
 template <int DIR>
-NMG_D void plain_directional(const EncodingParams& e, const float* xs, float* act, int n_grid, int r, int part) {
+NMG_D void plain_directional(const EncodingParams& e, const float* xs, float* act, int n_grid, int r, int h) {
   auto x = [&](int d) { return xs[d * kPlainRows + r]; };
   if constexpr (DIR == 0) {
-    if (part != 3) return;
+    if (h != 3) return;
     float xr[10], rest[64];
     for (int d = 0; d < 10; ++d) xr[d] = d < e.n_input ? x(d) : 0.f;
     encode_directional(e, xr, rest);
@@ -136,59 +141,54 @@ NMG_D void plain_directional(const EncodingParams& e, const float* xs, float* ac
   } else {
     constexpr int SH = DIR == 1 ? 4 : 2, SH2 = SH * SH;
     float* o = act + n_grid * kPlainRows + r;
-    if (part == 0 || (DIR == 1 && part == 1)) {
-      const int b = part == 0 ? 3 : 6;
+    if (h == 0 || (DIR == 1 && h == 1)) {
+      const int b = h == 0 ? 3 : 6;
       float d[16];
       sh_basis(SH, x(b) * 2.f - 1.f, x(b + 1) * 2.f - 1.f, x(b + 2) * 2.f - 1.f, d);
 #pragma unroll
-      for (int k = 0; k < SH2; ++k) o[(part * SH2 + k) * kPlainRows] = d[k];
-    } else if (DIR == 1 && part == 2) {
+      for (int k = 0; k < SH2; ++k) o[(h * SH2 + k) * kPlainRows] = d[k];
+    } else if (DIR == 2 || h == 2) {
       float d[4];
-      oneblob(4, x(9), d);
+      oneblob(4, x(DIR == 1 ? 9 : 5 + h), d);
 #pragma unroll
-      for (int k = 0; k < 4; ++k) o[(2 * SH2 + k) * kPlainRows] = d[k];
-    } else if (DIR == 1) {
-      for (int k = n_grid + 2 * SH2 + 4; k < e.n_enc_pad; ++k) act[k * kPlainRows + r] = 1.f;
-    } else {
-      float d[4];
-      oneblob(4, x(5 + part), d);
-#pragma unroll
-      for (int k = 0; k < 4; ++k) o[(SH2 + 4 * (part - 1) + k) * kPlainRows] = d[k];
-      if (part == 3)
-        for (int k = n_grid + SH2 + 12; k < e.n_enc_pad; ++k) act[k * kPlainRows + r] = 1.f;
+      for (int k = 0; k < 4; ++k) o[((DIR == 1 ? 2 * SH2 : SH2 + 4 * (h - 1)) + k) * kPlainRows] = d[k];
     }
+    if (h == 3)
+      for (int k = n_grid + (DIR == 1 ? 2 * SH2 + 4 : SH2 + 12); k < e.n_enc_pad; ++k) act[k * kPlainRows + r] = 1.f;
   }
 }
 
-// Thread tile of the matrix products: 4 rows x 4 columns. A warp covers 16
-// rows x 32 columns, so that each of its two 16-byte shared loads per step is
-// one wavefront; the block covers 64 x 64 at a time.
+// The product warps' thread tile: 4 rows x 8 columns, a warp 32 rows x 32
+// columns, the four warps 64 x 64.
 struct PlainTile {
   int row, col;
   NMG_D PlainTile() {
     const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    row = 16 * (wid & 3) + 4 * (lane & 3);
-    col = 32 * (wid >> 2) + 4 * (lane >> 2);
+    row = 32 * (wid & 1) + 4 * (lane & 7);
+    col = 32 * ((wid >> 1) & 1) + 8 * (lane >> 3);
   }
 };
 
 // acc[column][row] = sum over k < n of A[k][row] B[k][col], k ascending.
-NMG_D void plain_product(const float* A, const float* B, int ldb, int n, float (&acc)[4][4]) {
+NMG_D void plain_product(const float* A, const float* B, int ldb, int n, float (&acc)[8][4]) {
 #pragma unroll
-  for (int c = 0; c < 4; ++c)
+  for (int c = 0; c < 8; ++c)
 #pragma unroll
     for (int r = 0; r < 4; ++r) acc[c][r] = 0.f;
 #pragma unroll 4
   for (int k = 0; k < n; ++k) {
     const float4 a = *reinterpret_cast<const float4*>(A + k * kPlainRows);
-    const float4 b = *reinterpret_cast<const float4*>(B + k * ldb);
-    const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
+    const float4 b = *reinterpret_cast<const float4*>(B + k * ldb), b2 = *reinterpret_cast<const float4*>(B + k * ldb + 4);
+    const float av[4] = {a.x, a.y, a.z, a.w}, bv[8] = {b.x, b.y, b.z, b.w, b2.x, b2.y, b2.z, b2.w};
 #pragma unroll
-    for (int c = 0; c < 4; ++c)
+    for (int c = 0; c < 8; ++c)
 #pragma unroll
       for (int r = 0; r < 4; ++r) acc[c][r] = fmaf(av[r], bv[c], acc[c][r]);
   }
 }
+
+NMG_D void bar_product() { asm volatile("bar.sync 1, %0;" ::"n"(kProduct) : "memory"); }
+NMG_D void bar_movers() { asm volatile("bar.sync 2, %0;" ::"n"(kMovers) : "memory"); }
 
 constexpr int kPlainPad = 4;  // floats after each transposed weight row: its 16-byte stores spread over the banks
 
@@ -214,31 +214,35 @@ __global__ void __launch_bounds__(kPlainThreads, 2) k_plain_forward(const __grid
     }
     w_floats += nin * ld;
   }
-  float* act = sm + w_floats;                                    // [max(n_enc, 64)][64]
-  float* xs = act + (n_enc > kWidth ? n_enc : kWidth) * kPlainRows;  // [10][64]
+  const int act_floats = (n_enc > kWidth ? n_enc : kWidth) * kPlainRows;
+  float* act = sm + w_floats;          // two buffers of [max(n_enc, 64)][64]
+  float* xs = act + 2 * act_floats;    // [10][64]
   const int n = plain_count(p);
-  const int r = threadIdx.x % kPlainRows, part = threadIdx.x / kPlainRows;
+  const bool encoder = threadIdx.x >= kProduct;
+  const int t = int(threadIdx.x) - kProduct, r = t % kPlainRows, h = t / kPlainRows;  // of an encoder
   const PlainTile tl;
   const int tiles = (n + kPlainRows - 1) / kPlainRows;
-  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+
+  // One tile's rows into A (the encoder warps; two threads per row, which take
+  // every second level each).
+  auto encode = [&](int tile, float* A) {
     const long q0 = long(tile) * kPlainRows, q = q0 + r;
-    __syncthreads();
     if (a.in.pos) {
       if (q < n) {
-        featurize_part(p.enc, a.in, q, part, r, xs);
-      } else if (part == 0) {
+        featurize_part(p.enc, a.in, q, 2 * h, r, xs);
+        featurize_part(p.enc, a.in, q, 2 * h + 1, r, xs);
+      } else if (h == 0) {
         for (int d = 0; d < p.enc.n_input; ++d) xs[d * kPlainRows + r] = 0.f;
       }
     } else {
       const int ni = p.enc.n_input;
-      for (int i = threadIdx.x; i < kPlainRows * ni; i += kPlainThreads) {
+      for (int i = t; i < kPlainRows * ni; i += kMovers) {
         const int rr = i / ni, d = i - rr * ni;
         xs[d * kPlainRows + rr] = q0 + rr < n ? a.x[q0 * ni + i] : 0.f;
       }
     }
-    __syncthreads();
-    // ---- encoding: the row's four threads take every fourth level each
-    for (int l = part; l < p.enc.levels; l += 4) {
+    bar_movers();
+    for (int l = h; l < p.enc.levels; l += 2) {
       float w[3];
       uint32_t g[3];
 #pragma unroll
@@ -256,51 +260,66 @@ __global__ void __launch_bounds__(kPlainThreads, 2) k_plain_forward(const __grid
         for (int f = 0; f < F; ++f) acc[f] = fmaf(wt, v[f], acc[f]);
       }
 #pragma unroll
-      for (int f = 0; f < F; ++f) act[(l * F + f) * kPlainRows + r] = acc[f];
+      for (int f = 0; f < F; ++f) A[(l * F + f) * kPlainRows + r] = acc[f];
     }
-    plain_directional<DIR>(p.enc, xs, act, n_grid, r, part);
-    __syncthreads();
+    plain_directional<DIR>(p.enc, xs, A, n_grid, r, 2 * h);
+    plain_directional<DIR>(p.enc, xs, A, n_grid, r, 2 * h + 1);
+    bar_movers();  // xs is rewritten by the next call
     if (a.enc_t) {
       float4* dst = reinterpret_cast<float4*>(a.enc_t + size_t(tile) * kPlainRows * n_enc);
-      for (int i = threadIdx.x; i < n_enc * kPlainRows / 4; i += kPlainThreads)
-        dst[i] = reinterpret_cast<const float4*>(act)[i];
+      for (int i = t; i < n_enc * kPlainRows / 4; i += kMovers) dst[i] = reinterpret_cast<const float4*>(A)[i];
     }
-    // ---- layers
+  };
+
+  // One tile's layers, in place in A (the product warps).
+  auto layers = [&](int tile, float* A) {
+    const long q0 = long(tile) * kPlainRows;
     const float* Wl = W;
     for (int l = 0; l < L; ++l) {
       const int nin = p.in[l], nout = p.out[l], ld = nout + kPlainPad;
-      float acc[4][4];
+      float acc[8][4];
       if (l == L - 1) {
         for (int c0 = tl.col; c0 < nout; c0 += kWidth) {
-          plain_product(act + tl.row, Wl + c0, ld, nin, acc);
+          plain_product(A + tl.row, Wl + c0, ld, nin, acc);
 #pragma unroll
           for (int i = 0; i < 4; ++i)
             if (q0 + tl.row + i < n) {
               float* dst = a.raw + (q0 + tl.row + i) * a.ld_raw + c0;
               if (a.raw_wide) {
                 *reinterpret_cast<float4*>(dst) = make_float4(acc[0][i], acc[1][i], acc[2][i], acc[3][i]);
+                *reinterpret_cast<float4*>(dst + 4) = make_float4(acc[4][i], acc[5][i], acc[6][i], acc[7][i]);
               } else {
 #pragma unroll
-                for (int c = 0; c < 4; ++c) dst[c] = acc[c][i];
+                for (int c = 0; c < 8; ++c) dst[c] = acc[c][i];
               }
             }
         }
         break;
       }
-      plain_product(act + tl.row, Wl + tl.col, ld, nin, acc);  // hidden layers are kWidth wide
-      __syncthreads();
+      plain_product(A + tl.row, Wl + tl.col, ld, nin, acc);  // hidden layers are kWidth wide
+      bar_product();
       float* keep = a.h_t[l] ? a.h_t[l] + size_t(tile) * kPlainRows * kWidth : nullptr;
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
+      for (int c = 0; c < 8; ++c) {
         const float4 v = make_float4(fmaxf(acc[c][0], 0.f), fmaxf(acc[c][1], 0.f), fmaxf(acc[c][2], 0.f),
                                      fmaxf(acc[c][3], 0.f));
         const int at = (tl.col + c) * kPlainRows + tl.row;
-        *reinterpret_cast<float4*>(act + at) = v;
+        *reinterpret_cast<float4*>(A + at) = v;
         if (keep) *reinterpret_cast<float4*>(keep + at) = v;
       }
-      __syncthreads();
+      bar_product();
       Wl += nin * ld;
     }
+  };
+
+  int buf = 0;
+  if (encoder && int(blockIdx.x) < tiles) encode(blockIdx.x, act);
+  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, buf ^= 1) {
+    __syncthreads();
+    if (!encoder)
+      layers(tile, act + buf * act_floats);
+    else if (tile + int(gridDim.x) < tiles)
+      encode(tile + gridDim.x, act + (buf ^ 1) * act_floats);
   }
 }
 
@@ -336,106 +355,118 @@ NMG_D void plain_scatter(const PlainNet& p, int l, const float (&pos)[3], const 
 }
 
 // Deltas of every layer from dL/draw, and the grid gradient. Of layer 0's
-// input only the grid columns have parameters below.
+// input only the grid columns have parameters below. The product warps carry
+// one tile's delta from the last layer to the first in D and leave its grid
+// gradient in G; the other warps meanwhile scatter the last tile's grid
+// gradient and read the next tile's dL/draw (both buffers are double).
 template <int F>
 __global__ void __launch_bounds__(kPlainThreads, 2) k_plain_backward(const __grid_constant__ PlainBwd a) {
   extern __shared__ __align__(16) float sm[];
   const PlainNet& p = a.net;
-  const int L = p.n_layers, nout = p.out[L - 1], g4 = (p.n_grid + 3) / 4 * 4;
-  float* W = sm;  // per layer, the last first: [out][in], layer 0: [out][g4]
+  const int L = p.n_layers, nout = p.out[L - 1], ng = (p.n_grid + 15) / 16 * 16;
+  float* W = sm;  // per layer, the last first: [out][in], layer 0: [out][ng]
   int w_floats = 0;
   for (int l = L - 1; l >= 0; --l) {
-    const int ld = l == 0 ? g4 : p.in[l];
+    const int ld = l == 0 ? ng : p.in[l];
     for (int i = threadIdx.x; i < p.out[l] * (ld / 4); i += kPlainThreads) {
       const int j = i / (ld / 4), k = i - j * (ld / 4);
       reinterpret_cast<float4*>(W + w_floats)[i] = __ldg(reinterpret_cast<const float4*>(p.w[l] + size_t(j) * p.in[l]) + k);
     }
     w_floats += p.out[l] * ld;
   }
-  int dw = nout > kWidth ? nout : kWidth;
-  if (g4 > dw) dw = g4;
-  float* D = sm + w_floats;          // [dw][64]
-  float* xs = D + dw * kPlainRows;   // [3][64]
+  const int d_floats = (nout > kWidth ? nout : kWidth) * kPlainRows;
+  float* D = sm + w_floats;              // two buffers
+  float* G = D + 2 * d_floats;           // two buffers of [ng][64]
+  float* xs = G + 2 * ng * kPlainRows;   // two buffers of [3][64]
   const int n = plain_count(p), ni = p.enc.n_input;
+  const bool mover = threadIdx.x >= kProduct;
+  const int t = int(threadIdx.x) - kProduct;  // of a mover
   const PlainTile tl;
   const int tiles = (n + kPlainRows - 1) / kPlainRows;
-  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+
+  auto read = [&](int tile, int buf) {
     const long q0 = long(tile) * kPlainRows;
-    __syncthreads();
-    {
-      float* keep = a.d_t[L - 1] + size_t(tile) * kPlainRows * nout;
-      for (int i = threadIdx.x; i < kPlainRows * (nout / 4); i += kPlainThreads) {
-        const int r = i % kPlainRows, k = i / kPlainRows;
-        const float4 v = q0 + r < n ? __ldg(reinterpret_cast<const float4*>(a.draw + (q0 + r) * nout) + k)
-                                    : make_float4(0.f, 0.f, 0.f, 0.f);
-        const float e[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          D[(4 * k + c) * kPlainRows + r] = e[c];
-          keep[(4 * k + c) * kPlainRows + r] = e[c];
-        }
-      }
-      if (threadIdx.x < 3 * kPlainRows) {
-        const int r = threadIdx.x % kPlainRows, d = threadIdx.x / kPlainRows;
-        xs[threadIdx.x] = q0 + r < n ? a.x[(q0 + r) * ni + d] : 0.f;
-      }
-    }
-    __syncthreads();
-    const float* Wl = W;
-    float acc[4][4];
-    for (int l = L - 1; l >= 1; --l) {
-      const size_t at0 = size_t(tile) * kPlainRows * kWidth;
-      float4 h[4];
-#pragma unroll
-      for (int c = 0; c < 4; ++c)
-        h[c] = __ldg(reinterpret_cast<const float4*>(a.h_t[l - 1] + at0 + (tl.col + c) * kPlainRows + tl.row));
-      plain_product(D + tl.row, Wl + tl.col, kWidth, p.out[l], acc);
-      __syncthreads();
+    float* keep = a.d_t[L - 1] + size_t(tile) * kPlainRows * nout;
+    for (int i = t; i < kPlainRows * (nout / 4); i += kMovers) {
+      const int r = i % kPlainRows, k = i / kPlainRows;
+      const float4 v = q0 + r < n ? __ldg(reinterpret_cast<const float4*>(a.draw + (q0 + r) * nout) + k)
+                                  : make_float4(0.f, 0.f, 0.f, 0.f);
+      const float e[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
-        const float4 v = make_float4(h[c].x > 0.f ? acc[c][0] : 0.f, h[c].y > 0.f ? acc[c][1] : 0.f,
-                                     h[c].z > 0.f ? acc[c][2] : 0.f, h[c].w > 0.f ? acc[c][3] : 0.f);
+        D[buf * d_floats + (4 * k + c) * kPlainRows + r] = e[c];
+        keep[(4 * k + c) * kPlainRows + r] = e[c];
+      }
+    }
+    for (int i = t; i < 3 * kPlainRows; i += kMovers) {
+      const int r = i % kPlainRows, d = i / kPlainRows;
+      xs[buf * 3 * kPlainRows + i] = q0 + r < n ? a.x[(q0 + r) * ni + d] : 0.f;
+    }
+  };
+  auto scatter = [&](int tile, int buf) {  // two lanes per row, every second level
+    const int r = (t >> 1) % kPlainRows;
+    if (long(tile) * kPlainRows + r >= n) return;
+    const float* x = xs + buf * 3 * kPlainRows + r;
+    const float pos[3] = {x[0], x[kPlainRows], x[2 * kPlainRows]};
+    for (int l = t / (2 * kPlainRows); l < p.enc.levels; l += kMovers / (2 * kPlainRows)) {
+      float g[F];
+#pragma unroll
+      for (int f = 0; f < F; ++f) g[f] = G[(buf * ng + l * F + f) * kPlainRows + r];
+      plain_scatter<F>(p, l, pos, g, t & 1u, a.gtable, a.wide != 0);
+    }
+  };
+  auto deltas = [&](int tile, int buf) {
+    float acc[8][4];
+    float* d = D + buf * d_floats;
+    const float* Wl = W;
+    for (int l = L - 1; l >= 1; --l) {
+      const size_t at0 = size_t(tile) * kPlainRows * kWidth;
+      plain_product(d + tl.row, Wl + tl.col, kWidth, p.out[l], acc);
+      bar_product();
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
         const int at = (tl.col + c) * kPlainRows + tl.row;
-        *reinterpret_cast<float4*>(D + at) = v;
+        const float4 h = __ldg(reinterpret_cast<const float4*>(a.h_t[l - 1] + at0 + at));
+        const float4 v = make_float4(h.x > 0.f ? acc[c][0] : 0.f, h.y > 0.f ? acc[c][1] : 0.f,
+                                     h.z > 0.f ? acc[c][2] : 0.f, h.w > 0.f ? acc[c][3] : 0.f);
+        *reinterpret_cast<float4*>(d + at) = v;
         *reinterpret_cast<float4*>(a.d_t[l - 1] + at0 + at) = v;
       }
-      __syncthreads();
+      bar_product();
       Wl += p.out[l] * kWidth;
     }
-    // layer 0: at most 128 grid columns, in two rounds of 64
-    float acc2[4][4];
-    const bool c1 = tl.col < g4, c2 = tl.col + kWidth < g4;
-    if (c1) plain_product(D + tl.row, Wl + tl.col, g4, kWidth, acc);
-    if (c2) plain_product(D + tl.row, Wl + tl.col + kWidth, g4, kWidth, acc2);
-    __syncthreads();
+    for (int c0 = tl.col; c0 < ng; c0 += kWidth) {
+      plain_product(d + tl.row, Wl + c0, ng, kWidth, acc);
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      if (c1)
-        *reinterpret_cast<float4*>(D + (tl.col + c) * kPlainRows + tl.row) =
+      for (int c = 0; c < 8; ++c)
+        *reinterpret_cast<float4*>(G + (buf * ng + c0 + c) * kPlainRows + tl.row) =
             make_float4(acc[c][0], acc[c][1], acc[c][2], acc[c][3]);
-      if (c2)
-        *reinterpret_cast<float4*>(D + (tl.col + kWidth + c) * kPlainRows + tl.row) =
-            make_float4(acc2[c][0], acc2[c][1], acc2[c][2], acc2[c][3]);
     }
-    __syncthreads();
-    const int r = (threadIdx.x >> 1) % kPlainRows;
-    if (q0 + r < n) {
-      const float pos[3] = {xs[r], xs[kPlainRows + r], xs[2 * kPlainRows + r]};
-      for (int l = threadIdx.x / (2 * kPlainRows); l < p.enc.levels; l += kPlainThreads / (2 * kPlainRows)) {
-        float g[F];
-#pragma unroll
-        for (int f = 0; f < F; ++f) g[f] = D[(l * F + f) * kPlainRows + r];
-        plain_scatter<F>(p, l, pos, g, threadIdx.x & 1u, a.gtable, a.wide != 0);
-      }
+  };
+
+  int buf = 0, last = -1;
+  if (mover && int(blockIdx.x) < tiles) read(blockIdx.x, 0);
+  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, buf ^= 1) {
+    __syncthreads();  // D[buf] and xs[buf], and the last tile's G, are in place
+    if (!mover) {
+      deltas(tile, buf);
+    } else {
+      if (last >= 0) scatter(last, buf ^ 1);
+      bar_movers();  // xs[buf ^ 1] is rewritten only when every lane has read it
+      if (tile + int(gridDim.x) < tiles) read(tile + gridDim.x, buf ^ 1);
     }
+    last = tile;
   }
+  __syncthreads();
+  if (mover && last >= 0) scatter(last, buf ^ 1);
 }
 
 // dW[j][i] += sum over rows of delta[j][row] input[i][row] for one 64 x 64
 // block of one layer's matrix (blockIdx.y), over this block's share of the
-// tiles. Thread (j, i) = (8 lanes x 2 warps, 4 lanes x 4 warps) holds every
-// 16th row and column: a 16-byte shared load of four rows of a column is then
-// one wavefront (pitch 68 floats).
+// tiles. Four groups of 64 threads take 16 rows of a tile each; a thread holds
+// every 8th row and column of the 64 x 64 (8 x 8 sums, 16 shared loads per 256
+// FMAs; a 16-byte load of four rows of a column is conflict-free at a pitch of
+// 68 floats). The groups' sums meet in shared memory at the end.
 struct PlainWgradBlock {
   const float *d_t, *x_t;  // tiles [nout][64], [nin][64]
   float* dw;
@@ -449,68 +480,88 @@ struct PlainWgrad {
 };
 constexpr int kWgradPitch = kPlainRows + 4;
 
-__global__ void __launch_bounds__(kPlainThreads, 3) k_plain_wgrad(const __grid_constant__ PlainWgrad a) {
-  __shared__ __align__(16) float Ds[64 * kWgradPitch], Xs[64 * kWgradPitch];
+constexpr int kWgradThreads = 256, kWgradFloats = 2 * 64 * kWgradPitch;  // one stage: delta and input tile
+
+// 16 bytes global -> shared, or 16 zero bytes.
+NMG_D void copy16(float* dst, const float* src, bool valid) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(uint32_t(__cvta_generic_to_shared(dst))), "l"(src),
+               "r"(valid ? 16 : 0)
+               : "memory");
+}
+
+__global__ void __launch_bounds__(kWgradThreads, 2) k_plain_wgrad(const __grid_constant__ PlainWgrad a) {
+  extern __shared__ __align__(16) float sh[];  // two stages
   const PlainWgradBlock& b = a.blk[blockIdx.y];
   int n = a.n_max;
   if (a.d_count) n = *a.d_count < 0 ? 0 : (*a.d_count > n ? n : *a.d_count);
   const int tiles = (n + kPlainRows - 1) / kPlainRows;
+  if (int(blockIdx.x) >= tiles) return;
   const int nj = b.nout - b.j0 < 64 ? b.nout - b.j0 : 64, nx = b.nin - b.i0 < 64 ? b.nin - b.i0 : 64;
-  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int i = (lane & 7) + 8 * (wid & 1), j = (lane >> 3) + 4 * (wid >> 1);
-  float acc[4][4] = {};
-  // this thread's four 16-byte pieces of either tile (column c / 16, rows 4 (c % 16) ..)
-  float4 dv[4], xv[4];
-  auto fetch = [&](int tile) {
+  const int grp = threadIdx.x / 64, t = threadIdx.x % 64;
+  const int i = t & 7, j = t >> 3;
+  float acc[8][8] = {};
+  auto fetch = [&](int tile, int stage) {  // columns c / 16, rows 4 (c % 16) ..; columns beyond the matrix as zeros
     const float* d = b.d_t + (size_t(tile) * b.nout + b.j0) * kPlainRows;
     const float* x = b.x_t + (size_t(tile) * b.nin + b.i0) * kPlainRows;
+    float* s = sh + stage * kWgradFloats;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      const int c = threadIdx.x + k * kPlainThreads;
-      const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
-      dv[k] = c / 16 < nj ? __ldg(reinterpret_cast<const float4*>(d) + c) : z;
-      xv[k] = c / 16 < nx ? __ldg(reinterpret_cast<const float4*>(x) + c) : z;
+      const int c = threadIdx.x + k * kWgradThreads, at = (c / 16) * kWgradPitch + 4 * (c % 16);
+      copy16(s + at, c / 16 < nj ? d + 4 * c : d, c / 16 < nj);
+      copy16(s + 64 * kWgradPitch + at, c / 16 < nx ? x + 4 * c : x, c / 16 < nx);
     }
+    asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  int tile = blockIdx.x;
-  if (tile < tiles) fetch(tile);
-  for (; tile < tiles; tile += gridDim.x) {
-    __syncthreads();
+  int stage = 0;
+  fetch(blockIdx.x, 0);
+  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, stage ^= 1) {
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();  // this stage is in place, and the other one has been read
+    if (tile + int(gridDim.x) < tiles) fetch(tile + gridDim.x, stage ^ 1);
+    const float *Ds = sh + stage * kWgradFloats, *Xs = Ds + 64 * kWgradPitch;
+#pragma unroll 1
+    for (int r = 16 * grp; r < 16 * grp + 16; r += 4) {
+      float4 d[8];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int c = threadIdx.x + k * kPlainThreads;
-      *reinterpret_cast<float4*>(Ds + (c / 16) * kWgradPitch + 4 * (c % 16)) = dv[k];
-      *reinterpret_cast<float4*>(Xs + (c / 16) * kWgradPitch + 4 * (c % 16)) = xv[k];
-    }
-    __syncthreads();
-    if (tile + gridDim.x < tiles) fetch(tile + gridDim.x);
-    if (i < nx && j < nj) {
-#pragma unroll 2
-      for (int r = 0; r < kPlainRows; r += 4) {
-        float4 d[4], x[4];
+      for (int k = 0; k < 8; ++k) d[k] = *reinterpret_cast<const float4*>(Ds + (j + 8 * k) * kWgradPitch + r);
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          d[k] = *reinterpret_cast<const float4*>(Ds + (j + 16 * k) * kWgradPitch + r);
-          x[k] = *reinterpret_cast<const float4*>(Xs + (i + 16 * k) * kWgradPitch + r);
+      for (int v = 0; v < 8; ++v) {
+        if (8 * v >= nx) break;  // the block's columns beyond the matrix
+        const float4 x = *reinterpret_cast<const float4*>(Xs + (i + 8 * v) * kWgradPitch + r);
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          acc[u][v] = fmaf(d[u].x, x.x, acc[u][v]);
+          acc[u][v] = fmaf(d[u].y, x.y, acc[u][v]);
+          acc[u][v] = fmaf(d[u].z, x.z, acc[u][v]);
+          acc[u][v] = fmaf(d[u].w, x.w, acc[u][v]);
         }
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-#pragma unroll
-          for (int v = 0; v < 4; ++v) {
-            acc[u][v] = fmaf(d[u].x, x[v].x, acc[u][v]);
-            acc[u][v] = fmaf(d[u].y, x[v].y, acc[u][v]);
-            acc[u][v] = fmaf(d[u].z, x[v].z, acc[u][v]);
-            acc[u][v] = fmaf(d[u].w, x[v].w, acc[u][v]);
-          }
       }
     }
   }
-  if (int(blockIdx.x) >= tiles) return;
+  // groups 1-3 hand their sums to group 0 one after another
+  for (int g = 3; g >= 1; --g) {
+    __syncthreads();
 #pragma unroll
-  for (int u = 0; u < 4; ++u)
+    for (int u = 0; u < 8; ++u)
 #pragma unroll
-    for (int v = 0; v < 4; ++v) {
-      const int jj = j + 16 * u, ii = i + 16 * v;
+      for (int v = 0; v < 8; ++v) {
+        float& s = sh[(u * 8 + v) * 64 + t];
+        if (grp == g) s = acc[u][v];
+      }
+    __syncthreads();
+    if (grp == 0) {
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+#pragma unroll
+        for (int v = 0; v < 8; ++v) acc[u][v] += sh[(u * 8 + v) * 64 + t];
+    }
+  }
+  if (grp != 0) return;
+#pragma unroll
+  for (int u = 0; u < 8; ++u)
+#pragma unroll
+    for (int v = 0; v < 8; ++v) {
+      const int jj = j + 8 * u, ii = i + 8 * v;
       if (jj < nj && ii < nx) atomicAdd(b.dw + size_t(b.j0 + jj) * b.nin + b.i0 + ii, acc[u][v]);
     }
 }
@@ -579,7 +630,7 @@ nmg_status plain_forward(nmg_ctx* c, const nmg_shading* in, const float* x, cons
     for (int l = 0; l < c->lay.n_layers - 1; ++l) a.h_t[l] = w.h[l];
   }
   const int ne = c->enc.n_enc_pad;
-  size_t fl = size_t(ne > kWidth ? ne : kWidth) * kPlainRows + 10 * kPlainRows;
+  size_t fl = 2 * size_t(ne > kWidth ? ne : kWidth) * kPlainRows + 10 * kPlainRows;
   for (int l = 0; l < c->lay.n_layers; ++l) fl += size_t(c->lay.in[l]) * (c->lay.out[l] + kPlainPad);
   const size_t smem = fl * sizeof(float);
   const EncodingParams& e = c->enc;
@@ -620,10 +671,8 @@ nmg_status plain_backward(nmg_ctx* c, const float* x, const int* d_count, int n_
   }
   a.gtable = dparams + L.n_mlp;
   a.wide = aligned16(a.gtable);
-  const int g4 = (a.net.n_grid + 3) / 4 * 4;
-  int dw = L.n_out_pad > kWidth ? L.n_out_pad : kWidth;
-  if (g4 > dw) dw = g4;
-  size_t fl = size_t(dw) * kPlainRows + 3 * kPlainRows + size_t(kWidth) * g4;
+  const int ng = (a.net.n_grid + 15) / 16 * 16, dw = L.n_out_pad > kWidth ? L.n_out_pad : kWidth;
+  size_t fl = 2 * size_t(dw + ng) * kPlainRows + 6 * kPlainRows + size_t(kWidth) * ng;
   for (int l = 1; l < L.n_layers; ++l) fl += size_t(L.in[l]) * L.out[l];
   const size_t smem = fl * sizeof(float);
   switch (c->enc.feats) {
@@ -643,11 +692,13 @@ nmg_status plain_backward(nmg_ctx* c, const float* x, const int* d_count, int n_
                                       L.out[l], L.in[l], j0, i0};
   g.d_count = d_count;
   g.n_max = n_max;
-  // three blocks per SM in all; each adds its 64 x 64 sums once
+  // two blocks per SM in all; each adds its 64 x 64 sums once
   const long tiles = (long(n_max) + kPlainRows - 1) / kPlainRows;
-  long gx = (3L * sm_count() + nb - 1) / nb;
+  long gx = 2L * sm_count() / nb;
   if (gx > tiles) gx = tiles;
-  k_plain_wgrad<<<dim3(unsigned(gx < 1 ? 1 : gx), unsigned(nb)), kPlainThreads, 0, st>>>(g);
+  const size_t wsm = 2 * kWgradFloats * sizeof(float);
+  NMG_TRY(ensure_smem(reinterpret_cast<const void*>(k_plain_wgrad), wsm));
+  k_plain_wgrad<<<dim3(unsigned(gx < 1 ? 1 : gx), unsigned(nb)), kWgradThreads, wsm, st>>>(g);
   return check_launch("k_plain_wgrad");
 }
 
