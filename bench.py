@@ -651,13 +651,12 @@ def train_frame_row(nmg, torch, cfg, recs, cur, res, timed):
 def launches_per_step(path):
     """Kernels of this library launched per timed step (query pass + train step)."""
     if path == 0:
-        # query: featurize, encode, 4 linear, mixture; train: encode, 4 linear, loss, 4x(wgrad+dgrad),
-        # grid scatter, step counter, adam, stats
-        return 7 + (1 + 4 + 1 + 8 + 1 + 1 + 1 + 1)
+        # query: network, mixture; train: network forward, loss, network backward, weight gradient, adam, finish
+        return 2 + 6
     return 1 + FUSED_TRAIN_LAUNCHES
 
 
-FUSED_TRAIN_LAUNCHES = 5  # k_fused_train, k_step_inc, k_adam_ema, k_finish_stats, k_pack_weights
+FUSED_TRAIN_LAUNCHES = 3  # k_fused_train, k_adam_ema, k_finish_step
 
 
 def cpu_baseline(q, x, rec, seconds=15.0, kind="port"):

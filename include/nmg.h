@@ -354,12 +354,15 @@ nmg_status nmg_network_vjp(nmg_ctx* ctx, const float* x, const float* draw, int 
 /*
  * Tiling of the fused query kernel: warpgroups (128-query tiles in flight)
  * per CTA, one CTA per SM; 5 and 6 are valid when the padded output width is
- * <= 64. 7: two tiles in flight, each on two warpgroups, two threads per
- * query splitting the lobes (queries that return raw outputs fall back to
- * 4). 8-12 select configurations of the warp-specialised kernel: encoder
- * warpgroups feed MLP + mixture warpgroups through a shared-memory ring
- * (8: 4 + 2 warpgroups, 4 slots; 9: 5 + 1, 5 slots; 10: 6 + 2, 6 slots;
- * 11: 4 + 2, 8 slots; 12: 4 + 2, 4 slots holding the hidden activations too).
+ * <= 64. 7: for 8-lobe networks two tiles in flight, each on two warpgroups,
+ * two threads per query splitting the lobes (queries that return raw outputs
+ * fall back to 4); for 16-lobe networks encoder, MLP and mixture warpgroups,
+ * four threads per query in the mixture. 8-12 select warp-specialised kernels:
+ * 12 encoder, MLP and mixture warpgroups, 8 (8-lobe networks) warpgroups that
+ * encode and run the MLP, and mixture warpgroups; in the others (and 8 at 16
+ * lobes: 4 + 2 warpgroups, 4 slots) encoder warpgroups feed MLP + mixture
+ * warpgroups through a shared-memory ring (9: 5 + 1, 5 slots; 10: 6 + 2, 6
+ * slots; 11: 4 + 2, 8 slots).
  * 0 selects the default: 12 for the 8-lobe hash-grid network, 8 for the
  * reference network, 7 for 16-lobe networks. A tiling whose shared memory
  * exceeds the device's limit for this network's weight image makes the

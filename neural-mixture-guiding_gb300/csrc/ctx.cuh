@@ -90,7 +90,8 @@ nmg_status plain_train_step(nmg_ctx* c, const float* x, const float* rec, const 
                             double* stats, cudaStream_t st);
 nmg_status plain_vjp(nmg_ctx* c, const float* x, const float* draw, int n, float* raw, float* dparams,
                      cudaStream_t st);
-nmg_status optimizer_step(nmg_ctx* c, const int* d_count, int n_max, double* stats, cudaStream_t st);
+// n_loss: blocks that left a loss partial in ws.partials. Ends with the weight images and cell records refreshed.
+nmg_status optimizer_step(nmg_ctx* c, const int* d_count, int n_max, int n_loss, double* stats, cudaStream_t st);
 nmg_status init_params(nmg_ctx* c, uint32_t seed, cudaStream_t st);
 nmg_status sync_copies(nmg_ctx* c, cudaStream_t st);
 
@@ -103,6 +104,8 @@ nmg_status fused_infer_raw(nmg_ctx* c, const float* x, const int* d_count, int n
 nmg_status fused_pdf(nmg_ctx* c, const nmg_shading* in, const float* wi, const int* d_count, int n_max, float* pdf,
                      cudaStream_t st);
 nmg_status pack_images(nmg_ctx* c, cudaStream_t st);
+nmg_status finish_step(nmg_ctx* c, const double* loss, int n_loss, const double* norm, int n_norm, const int* d_count,
+                       int n_max, double* stats, uint32_t* step, cudaStream_t st);
 void fused_release(nmg_ctx* c);
 nmg_status fused_check_errors(nmg_ctx* c);
 nmg_status fused_selftest_wait_timeout(nmg_ctx* c, cudaStream_t st);

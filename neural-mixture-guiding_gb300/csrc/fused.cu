@@ -26,6 +26,7 @@
 #include <sys/stat.h>
 
 #include <string>
+#include <type_traits>
 
 #include "api_common.cuh"
 #include "ctx.cuh"
@@ -161,7 +162,7 @@ __global__ void __launch_bounds__(NWG * kRows, 1) k_fused_query(const __grid_con
   }
 }
 
-// Tiling 7: two pipelines per CTA, each two warpgroups on one 128-query tile
+// Tiling 7 of the 8-lobe networks: two pipelines per CTA, each two warpgroups on one 128-query tile
 // (the layout of the training kernel): warps w and w + 4 read the same TMEM
 // lane quadrant, so every query has two threads, which split the encoding's
 // grid levels, each hidden epilogue's columns and the mixture's lobes. With
@@ -421,36 +422,135 @@ __global__ void __launch_bounds__(4 * kRows, 1) k_fused_query_pair(const __grid_
   }
 }
 
-// ------------------------------------------------------------ weight image
+// ------------------------------------------------- after the optimiser step
 // Element (n, k) of layer l goes to byte layer_off[l] + cm_offset(n, k/8,
 // in_l/8) + 2 (k % 8): each layer becomes a K-major operand of N = out_l rows,
 // converted from the FP32 weights to the layer's operand format (PackArgs).
 // W0's low parts, bf16(w - bf16(w)), go to the same place relative to
-// w0_lo_off. blockIdx.y selects the image: 0 the training weights, 1 the
-// inference ones.
-__global__ void k_pack_weights(PackArgs p, const float* __restrict__ w_train, uint16_t* __restrict__ img_train,
-                               const float* __restrict__ w_infer, uint16_t* __restrict__ img_infer) {
-  const int which = blockIdx.y;
-  const float* __restrict__ w = which ? w_infer : w_train;
-  uint16_t* __restrict__ img = which ? img_infer : img_train;
-  const uint32_t fp16_layers = p.fp16_layers[which], lo_off = p.w0_lo_off[which];
-  const long total = p.off[p.n_layers];
-  for (long i = long(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += long(gridDim.x) * blockDim.x) {
-    int l = 0;
-    while (l + 1 < p.n_layers && i >= p.off[l + 1]) ++l;
-    const long j = i - p.off[l];
-    const int in = p.in[l];
-    const int nrow = int(j / in), k = int(j % in);
-    const uint32_t b = tc::cm_offset(nrow, k >> 3, in >> 3) + uint32_t(k & 7) * 2u;
-    const float v = w[i];
-    if ((fp16_layers >> l) & 1u) {
-      img[(p.layer_off[l] + b) >> 1] = __half_as_ushort(__float2half_rn(v));
+// w0_lo_off. Element i of image `which` (0 the training weights, 1 the
+// inference ones).
+NMG_D void pack_weight(const PackArgs& p, int which, long i, const float* __restrict__ w, uint16_t* __restrict__ img) {
+  const uint32_t lo_off = p.w0_lo_off[which];
+  int l = 0;
+  while (l + 1 < p.n_layers && i >= p.off[l + 1]) ++l;
+  const long j = i - p.off[l];
+  const int in = p.in[l];
+  const int nrow = int(j / in), k = int(j % in);
+  const uint32_t b = tc::cm_offset(nrow, k >> 3, in >> 3) + uint32_t(k & 7) * 2u;
+  const float v = w[i];
+  if ((p.fp16_layers[which] >> l) & 1u) {
+    img[(p.layer_off[l] + b) >> 1] = __half_as_ushort(__float2half_rn(v));
+  } else {
+    const __nv_bfloat16 hi = __float2bfloat16_rn(v);
+    img[(p.layer_off[l] + b) >> 1] = __bfloat16_as_ushort(hi);
+    if (l == 0 && lo_off)
+      img[(lo_off + b) >> 1] = __bfloat16_as_ushort(__float2bfloat16_rn(v - __bfloat162float(hi)));
+  }
+}
+
+// Cell record r from the 16-bit table.
+template <int F>
+NMG_D void pack_cell(const CellPackArgs& p, uint32_t r, const uint16_t* __restrict__ table16, uint4* __restrict__ cells) {
+  using Entry = typename std::conditional<F == 2, uint32_t, uint2>::type;  // F 16-bit features
+  int i = 0;
+  while (r >= p.first[i + 1]) ++i;
+  const uint32_t c = r - p.first[i], T = p.T[i], res = p.res[i];
+  const bool oct = (p.oct_mask >> i) & 1u;
+  const Entry* tab = reinterpret_cast<const Entry*>(table16) + p.table_off[i];
+  uint32_t w[8];
+#pragma unroll
+  for (int k = 0; k < (F == 2 ? 8 : 4); ++k) {
+    if (k >= 4 && !oct) break;
+    const uint32_t off = oct ? uint32_t(k & 1) + uint32_t((k >> 1) & 1) * res + uint32_t(k >> 2) * res * res
+                             : uint32_t(k & 1) * res + uint32_t(k >> 1) * res * res;
+    uint32_t idx = c + off;
+    if (idx >= T) idx %= T;
+    const Entry e = tab[idx];
+    if constexpr (F == 2) {
+      w[k] = e;
     } else {
-      const __nv_bfloat16 hi = __float2bfloat16_rn(v);
-      img[(p.layer_off[l] + b) >> 1] = __bfloat16_as_ushort(hi);
-      if (l == 0 && lo_off)
-        img[(lo_off + b) >> 1] = __bfloat16_as_ushort(__float2bfloat16_rn(v - __bfloat162float(hi)));
+      w[2 * k] = e.x;
+      w[2 * k + 1] = e.y;
     }
+  }
+  const bool wide = F == 4 || oct;
+  uint4* dst = cells + p.cell_off[i] + size_t(c) * (wide ? 2 : 1);
+  dst[0] = make_uint4(w[0], w[1], w[2], w[3]);
+  if (wide) dst[1] = make_uint4(w[4], w[5], w[6], w[7]);
+}
+
+// Everything that follows an optimiser step, in one launch (it was four: the
+// step counter, the statistics, the weight images, the cell records; each is
+// short, and a training step of a small batch is mostly such launches). Block
+// 0: stats[0] = sum of the loss partials / n, stats[1] = sqrt(sum of the
+// gradient-norm partials), both 0 for an empty batch, whose gradient-norm
+// partials are stale, and the step counter, which an empty batch leaves as it
+// is (see k_adam_ema). The other blocks, if any: both weight images, then both
+// copies' cell records, one element per thread, from the parameters and the
+// table that the step has just written (L2-resident).
+struct FinishArgs {
+  const double *loss, *norm;
+  int n_loss, n_norm;
+  const int* d_count;
+  int n_max;
+  double* stats;   // may be NULL
+  uint32_t* step;  // may be NULL
+  PackArgs pack;
+  CellPackArgs cells;
+  const float* w[2];  // training, inference
+  uint16_t* img[2];
+  const uint16_t* table[2];
+  uint4* cell_mem[2];
+  int img_blocks;  // per image
+};
+constexpr int kFinishThreads = 256;
+
+NMG_D double finish_sum(double v, double* s) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+  if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = v;
+  __syncthreads();
+  double r = 0.0;
+  if (threadIdx.x == 0)
+    for (int w = 0; w < kFinishThreads / 32; ++w) r += s[w];
+  __syncthreads();
+  return r;
+}
+
+template <int F>
+__global__ void __launch_bounds__(kFinishThreads) k_finish_step(const __grid_constant__ FinishArgs a) {
+  if (blockIdx.x == 0) {
+    __shared__ double s[kFinishThreads / 32];
+    int n = a.n_max;
+    if (a.d_count) n = *a.d_count < 0 ? 0 : (*a.d_count > n ? n : *a.d_count);
+    if (a.stats) {
+      double l = 0.0, g = 0.0;
+#pragma unroll 4
+      for (int i = threadIdx.x; i < a.n_loss; i += kFinishThreads) l += a.loss[i];
+#pragma unroll 8
+      for (int i = threadIdx.x; i < a.n_norm; i += kFinishThreads) g += a.norm[i];
+      l = finish_sum(l, s);
+      g = finish_sum(g, s);
+      if (threadIdx.x == 0) {
+        a.stats[0] = n > 0 ? l / double(n) : 0.0;
+        a.stats[1] = n > 0 ? sqrt(g) : 0.0;
+      }
+    }
+    if (threadIdx.x == 0 && a.step && !(a.d_count && *a.d_count <= 0)) *a.step += 1;
+    return;
+  }
+  const long b = long(blockIdx.x) - 1;
+  if (b < 2 * a.img_blocks) {
+    const int which = b >= a.img_blocks;
+    const long i = (b - which * a.img_blocks) * kFinishThreads + threadIdx.x;
+    if (i < a.pack.off[a.pack.n_layers]) pack_weight(a.pack, which, i, a.w[which], a.img[which]);
+    return;
+  }
+  const uint32_t total = a.cells.first[a.cells.n_lvl];
+  const long r = (b - 2 * a.img_blocks) * kFinishThreads + threadIdx.x;
+  if (r < 2 * long(total)) {
+    const int which = r >= total;
+    pack_cell<F>(a.cells, uint32_t(which ? r - total : r), a.table[which], a.cell_mem[which]);
   }
 }
 
@@ -522,17 +622,13 @@ static nmg_status launch_query_pair(const FusedArgs& a, cudaStream_t st) {
   return check_launch("k_fused_query_pair");
 }
 
-// Default query tiling: the warp-specialised kernel (4 encoder + 2 consumer
-// warpgroups) for the 8-lobe networks, measured 1.3x faster than one
-// pipeline per warpgroup on a 2,073,600-query wavefront; for the hash-grid
-// network its variant with the hidden activations kept in the ring slot
-// (tiling 12: 32 KB more L1 for the table gathers) measured 630 us against
-// 646 us. The 16-lobe network's consumer epilogue does not fit 128
-// registers: it takes tiling 7, two threads per query with 8 lobes each in
-// registers, 1.096 ms on a 2,073,600-query wavefront against 1.266 ms for one
-// pipeline per warpgroup re-deriving the lobes from TMEM and 1.344 ms for the
-// warp-specialised kernel (for 8 lobes tiling 7 measured 0.952 ms against
-// 0.643 ms for tiling 12).
+// Default query tiling: the kernels that give the mixture warpgroups of its own
+// (fused_ws.cu). Three roles for the hash-grid networks: tiling 12 at 8 lobes,
+// 535 us for a 2,073,600-query wavefront (one warpgroup for MLP and mixture:
+// 624 us; one pipeline per warpgroup: 759 us), tiling 7 at 16 lobes, 330 us for
+// 900,000 queries (two threads per query: 464 us). Two roles for the reference
+// network, tiling 8, whose 8 levels gather in half the time: 110 us for the pdf
+// of 550,001 queries (three roles: 122 us, before 150 us).
 int fused_default_tiling(const nmg_ctx* c) {
   const FusedState* s = reinterpret_cast<const FusedState*>(c->ws.fused);
   if (!s) return 4;
@@ -543,10 +639,10 @@ int fused_default_tiling(const nmg_ctx* c) {
 static nmg_status dispatch_query(nmg_ctx* c, const FusedArgs& a, cudaStream_t st) {
   const int nwg = c->query_wg > 0 ? c->query_wg : fused_default_tiling(c);
   if (nwg >= kTilingWarpSpecialised) return launch_query_ws(fstate(c)->preset, nwg, a, st);
+  if (nwg == kTilingPair && fstate(c)->preset == 2) return launch_query_ws(2, kTilingPair, a, st);
   if (nwg == kTilingPair && !a.raw && !a.raw_mode) {
     switch (fstate(c)->preset) {
       case 1: return launch_query_pair<2, 16, 1, 4, 4, 8, 48, false>(a, st);
-      case 2: return launch_query_pair<2, 16, 1, 4, 4, 16, 80, false>(a, st);
       case 3: return launch_query_pair<4, 8, 0, 2, 4, 8, 48, true>(a, st);
     }
   }
@@ -558,12 +654,71 @@ static nmg_status dispatch_query(nmg_ctx* c, const FusedArgs& a, cudaStream_t st
   return set_error(NMG_ERR_UNSUPPORTED, "configuration has no fused kernel");
 }
 
+// The optimiser step's last launch (k_finish_step). loss / norm: the partial
+// sums of the step's statistics.
+nmg_status finish_step(nmg_ctx* c, const double* loss, int n_loss, const double* norm, int n_norm, const int* d_count,
+                       int n_max, double* stats, uint32_t* step, cudaStream_t st) {
+  FinishArgs a;
+  memset(&a, 0, sizeof(a));
+  a.loss = loss;
+  a.norm = norm;
+  a.n_loss = n_loss;
+  a.n_norm = n_norm;
+  a.d_count = d_count;
+  a.n_max = n_max;
+  a.stats = stats;
+  a.step = step;
+  long blocks = 1;
+  const FusedState* s = fstate(c);
+  if (s) {
+    a.pack = s->pack;
+    a.cells = s->cells;
+    a.w[0] = c->w;
+    a.w[1] = c->w_inf;
+    a.img[0] = reinterpret_cast<uint16_t*>(s->img_train);
+    a.img[1] = reinterpret_cast<uint16_t*>(s->img_infer);
+    a.table[0] = c->w16 + c->lay.n_mlp;
+    a.table[1] = c->w16_inf + c->lay.n_mlp;
+    a.cell_mem[0] = s->cell_mem[0];
+    a.cell_mem[1] = s->cell_mem[1];
+    a.img_blocks = ceil_div(s->pack.off[s->pack.n_layers], kFinishThreads);
+    blocks += 2 * a.img_blocks + ceil_div(2 * long(s->cells.first[s->cells.n_lvl]), kFinishThreads);
+  }
+  if (c->enc.feats == 4)
+    k_finish_step<4><<<unsigned(blocks), kFinishThreads, 0, st>>>(a);
+  else
+    k_finish_step<2><<<unsigned(blocks), kFinishThreads, 0, st>>>(a);
+  return check_launch("k_finish_step");
+}
+
 nmg_status pack_images(nmg_ctx* c, cudaStream_t st) {
-  FusedState* s = fstate(c);
-  if (!s) return NMG_OK;
-  k_pack_weights<<<dim3(64, 2), 256, 0, st>>>(s->pack, c->w, reinterpret_cast<uint16_t*>(s->img_train), c->w_inf,
-                                              reinterpret_cast<uint16_t*>(s->img_infer));
-  return check_launch("k_pack_weights");
+  if (!fstate(c)) return NMG_OK;
+  return finish_step(c, nullptr, 0, nullptr, 0, nullptr, 0, nullptr, nullptr, st);
+}
+
+// The dense levels that get cell records, and where.
+static void plan_cells(const nmg_ctx* c, FusedState& s) {
+  const EncodingParams& e = c->enc;
+  CellPackArgs& p = s.cells;
+  p.feats = e.feats;
+  for (int l = 0; l < e.levels; ++l) {
+    const uint32_t T = e.offset[l + 1] - e.offset[l];
+    const unsigned long long r = e.res[l];
+    if (e.grid_hash && r * r * r > T) break;  // hashed, as are all finer levels
+    const bool oct = e.feats == 2 && T <= kOctEntries;
+    const uint32_t units = T * (oct || e.feats == 4 ? 2u : 1u);
+    if ((size_t(s.cell_units) + units) * 16 > kCellBytes) break;
+    const int i = p.n_lvl++;
+    p.T[i] = T;
+    p.res[i] = e.res[l];
+    p.table_off[i] = e.offset[l];
+    p.cell_off[i] = s.cell_units;
+    p.first[i + 1] = p.first[i] + T;
+    if (oct) p.oct_mask |= 1u << i;
+    s.lvl_rec |= 1u << l;
+    if (oct) s.lvl_oct |= 1u << l;
+    s.cell_units += (units + 1u) & ~1u;  // 32-byte aligned
+  }
 }
 
 nmg_status fused_reserve(nmg_ctx* c) {
@@ -598,8 +753,11 @@ nmg_status fused_reserve(nmg_ctx* c) {
   s.pack.fp16_layers[1] = all_layers;
   s.pack.w0_lo_off[1] = 0;
   s.w_bytes_inf = s.w_bytes;
+  plan_cells(c, s);
   const size_t head = 256;
-  const size_t bytes = head + size_t(s.w_bytes) + size_t(s.w_bytes_inf);
+  const size_t img = (size_t(s.w_bytes) + size_t(s.w_bytes_inf) + 31) & ~size_t(31);
+  const size_t cell_bytes = size_t(s.cell_units) * 16;
+  const size_t bytes = head + img + 2 * cell_bytes;
   void* mem = nullptr;
   cudaError_t e = cudaMalloc(&mem, bytes);
   if (e != cudaSuccess) return set_error(NMG_ERR_OOM, "fused workspace: %s", cudaGetErrorString(e));
@@ -609,6 +767,8 @@ nmg_status fused_reserve(nmg_ctx* c) {
   hs->err = reinterpret_cast<int*>(mem);
   hs->img_train = reinterpret_cast<uint8_t*>(mem) + head;
   hs->img_infer = hs->img_train + s.w_bytes;
+  hs->cell_mem[0] = reinterpret_cast<uint4*>(hs->img_train + img);
+  hs->cell_mem[1] = hs->cell_mem[0] + s.cell_units;
   c->ws.fused_dev = mem;
   c->ws.fused = hs;
   c->ws.fused_bytes = bytes;
@@ -640,6 +800,20 @@ FusedArgs fused_make_args(nmg_ctx* c, bool infer_weights) {
     a.lvl_T[l] = T;
     const unsigned long long r = c->enc.res[l];
     if (c->enc.grid_hash && r * r * r > T) a.lvl_hash |= 1u << l;
+  }
+  a.lvl_rec = s->lvl_rec;
+  a.lvl_oct = s->lvl_oct;
+  a.cells = s->cell_mem[infer_weights ? 1 : 0];
+  for (int i = 0; i < s->cells.n_lvl; ++i) a.cell_off[i] = s->cells.cell_off[i];
+  {  // a level costs a thread about as many L2 requests as it has corner pairs: 4 and a bit, or 1 with records
+    const int L = c->enc.levels;
+    int total = 0, sum = 0, l = 0;
+    for (int i = 0; i < L; ++i) total += (a.lvl_rec >> i) & 1u ? 1 : 4;
+    while (l + 2 < L && (l == 0 || 2 * sum < total)) {
+      for (int i = l; i < l + 2; ++i) sum += (a.lvl_rec >> i) & 1u ? 1 : 4;
+      l += 2;
+    }
+    a.half_levels = l;
   }
   a.n_out = c->lay.n_out;
   a.n_out_pad = c->lay.n_out_pad;

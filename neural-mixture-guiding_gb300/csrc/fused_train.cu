@@ -68,20 +68,6 @@ struct TrainArgs {
   nmg_radiance_records rr;
 };
 
-// D[tmem] (+)= sum over STEPS 16-deep slices of A and B whose descriptors
-// advance by a_step / b_step bytes per slice. The descriptors are formed once
-// and stepped by adding to their address field: one thread issues all of the
-// CTA's MMAs, and building two descriptors per MMA cost it more than the MMAs
-// take.
-template <int STEPS>
-NMG_D void issue_steps(uint32_t tmem, uint64_t a, uint32_t a_step, uint64_t b, uint32_t b_step, uint32_t idesc,
-                       bool accumulate) {
-#pragma unroll
-  for (int kk = 0; kk < STEPS; ++kk)
-    tc::mma_f16(tmem, a + uint64_t(kk * (a_step >> 4)), b + uint64_t(kk * (b_step >> 4)), idesc,
-                (accumulate || kk > 0) ? 1u : 0u);
-}
-
 // A K-major tile (a_chunks chunks a row) times a weight image: forward
 // (b_mn = false, the image K-major, kin / 16 slices) or data gradient (the
 // image of `in_chunks` chunks a row read MN-major).
@@ -776,7 +762,6 @@ nmg_status fused_train_step_src(nmg_ctx* c, const float* x, const float* rec, co
   if (grid < 1) grid = 1;
   if (grid > c->ws.n_partials / 2) grid = c->ws.n_partials / 2;
   NMG_CUDA_TRY(cudaMemsetAsync(c->grad, 0, sizeof(float) * size_t(c->lay.n_params), st));
-  NMG_CUDA_TRY(cudaMemsetAsync(c->ws.partials, 0, sizeof(double) * (c->ws.n_partials / 2), st));
   nmg_status r;
   // the records mode is its own instantiation: the load stage of the plain
   // one stays free of the record code
@@ -797,9 +782,7 @@ nmg_status fused_train_step_src(nmg_ctx* c, const float* x, const float* rec, co
     default: return set_error(NMG_ERR_UNSUPPORTED, "configuration has no fused kernel");
   }
   if (r != NMG_OK) return r;
-  r = optimizer_step(c, d_count, n_max, stats, st);
-  if (r != NMG_OK) return r;
-  return pack_images(c, st);
+  return optimizer_step(c, d_count, n_max, grid, stats, st);
 }
 
 }  // namespace nmg

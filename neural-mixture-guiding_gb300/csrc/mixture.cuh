@@ -290,6 +290,14 @@ template <bool FAST> NMG_D float one_minus_exp_neg(float x) {
   return x * (1.f - x * (1.f / 2.f) * (1.f - x * (1.f / 3.f) * (1.f - x * (1.f / 4.f) *
              (1.f - x * (1.f / 5.f) * (1.f - x * (1.f / 6.f) * (1.f - x * (1.f / 7.f)))))));
 }
+// The same value with both forms evaluated and one selected (hardware
+// exponential): no branch to keep a thread's lobes from overlapping.
+NMG_D float one_minus_exp_neg_flat(float x) {
+  const float lo = x * (1.f - x * (1.f / 2.f) * (1.f - x * (1.f / 3.f) * (1.f - x * (1.f / 4.f) *
+                   (1.f - x * (1.f / 5.f) * (1.f - x * (1.f / 6.f) * (1.f - x * (1.f / 7.f)))))));
+  const float hi = 1.f - __expf(-x);
+  return x >= 0.5f ? hi : lo;
+}
 template <bool FAST> NMG_D f3 unit3(f3 a) {
   if (!FAST) return normalize3(a);
   const float n2 = dot3(a, a);
@@ -329,6 +337,12 @@ template <bool FAST> NMG_D float vmf_norm(float k) {
   if (k < NMG_EPS) return NMG_INV_4PI;
   const float den = FAST ? one_minus_exp_neg<true>(2.f * k) : (k < 0.5f ? -expm1f(-2.f * k) : 1.f - expf(-2.f * k));
   return xdiv<FAST>(k, NMG_TWO_PI * den);
+}
+
+// vmf_norm<true> and (below) prod_norm<true> without branches.
+NMG_D float vmf_norm_flat(float k) {
+  const float v = __fdividef(k, NMG_TWO_PI * one_minus_exp_neg_flat(2.f * k));
+  return k < NMG_EPS ? NMG_INV_4PI : v;
 }
 
 // distribution.h:85-98: activation of one query's raw outputs. `raw` points
@@ -389,7 +403,38 @@ NMG_D void mix_activate_regs(Mix<K>& m, const float (&raw)[N], int kappa_softplu
 template <bool FAST> NMG_D float prod_norm(float k) {
   return k < 1e-3f ? NMG_INV_4PI : xdiv<FAST>(k * NMG_INV_2PI, one_minus_exp_neg<FAST>(2.f * k));
 }
+NMG_D float prod_norm_flat(float k) {
+  const float v = __fdividef(k * NMG_INV_2PI, one_minus_exp_neg_flat(2.f * k));
+  return k < 1e-3f ? NMG_INV_4PI : v;
+}
 constexpr float kCosineKappa = 2.18853f;  // distribution.h:184-195
+
+// lobe_cosine<true> without branches, its sum of scaled means fused in a stated
+// order, so that a lobe's mean and weight are the same bit for bit whatever
+// the compiler would contract in the kernel at hand (a mean off by one unit
+// can turn the sampler's frame, and a weight the selected lobe): LOBE_FIRST
+// rounds the cosine lobe's product and adds the lobe's to it, as the 16-lobe
+// query always has, else the other way round, as the 8-lobe query has.
+template <bool LOBE_FIRST>
+NMG_D void lobe_cosine_flat(f3 mb, float nb, float& lam, float& kap, f3& mu, float& nrm) {
+  const float kb = kCosineKappa, ka = kap;
+  const f3 ma = mu;
+  f3 nm = LOBE_FIRST ? f3{fmaf(ma.x, ka, mb.x * kb), fmaf(ma.y, ka, mb.y * kb), fmaf(ma.z, ka, mb.z * kb)}
+                     : f3{fmaf(mb.x, kb, ma.x * ka), fmaf(mb.y, kb, ma.y * ka), fmaf(mb.z, kb, ma.z * ka)};
+  const float n2 = dot3(nm, nm);
+  const float rn = rsqrtf(n2);
+  float nk = n2 * rn;
+  const bool some = nk >= 1e-3f;
+  nm = f3{some ? nm.x * rn : ma.x, some ? nm.y * rn : ma.y, some ? nm.z * rn : ma.z};
+  nk = some ? nk : 0.f;
+  const float e = __expf(ka * (dot3(nm, ma) - 1.f) + kb * (dot3(nm, mb) - 1.f));
+  const float pk = prod_norm_flat(nk);
+  const float pa = ka < 1e-3f ? NMG_INV_4PI : nrm;
+  lam = __fdividef(pa * nb, pk) * e * lam;
+  kap = nk;
+  mu = nm;
+  nrm = pk;
+}
 
 // One lobe (lam, kap, mu, nrm = its vMF normaliser) times the cosine lobe of
 // concentration kb = kCosineKappa around the unit mean mb (nb = its product

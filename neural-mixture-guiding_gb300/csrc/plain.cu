@@ -115,12 +115,8 @@ __global__ void __launch_bounds__(128) k_train_loss(const float* __restrict__ ra
 // ---------------------------------------------------------------- optimiser
 // A training step whose device count is zero takes no optimiser step (the
 // reference's training loop stops before a batch below its minimum size,
-// integrator.cpp:670-671): the step counter, Adam and the EMA leave the
-// parameters and the optimiser state as they are.
-__global__ void k_step_inc(uint32_t* step, const int* d_count) {
-  if (d_count && *d_count <= 0) return;
-  *step += 1;
-}
+// integrator.cpp:670-671): the step counter (k_finish_step), Adam and the EMA
+// leave the parameters and the optimiser state as they are.
 
 // adam.h:47-119 + ema.h:62-75/102-145 in one pass over four parameters per
 // thread (128-bit loads and stores); also writes the reduced-precision copies
@@ -150,8 +146,8 @@ __global__ void __launch_bounds__(256) k_adam_ema(AdamArgs a, const float4* __re
                                                   uint4* __restrict__ psteps, float4* __restrict__ w_inf,
                                                   uint2* __restrict__ w16, uint2* __restrict__ w16_inf,
                                                   double* __restrict__ partials, const int* __restrict__ d_count) {
-  if (d_count && *d_count <= 0) return;  // an empty batch takes no step (see k_step_inc)
-  const uint32_t step = *d_step;
+  if (d_count && *d_count <= 0) return;  // an empty batch takes no step
+  const uint32_t step = *d_step + 1;  // d_step counts the steps taken before this one
   const float debias_old = 1.f - exp2f(float(step - 1) * a.log2_decay);
   const float debias_new = 1.f / (1.f - exp2f(float(step) * a.log2_decay));
   const bool separate_inf = w_inf != w;
@@ -211,28 +207,6 @@ __global__ void __launch_bounds__(256) k_adam_ema(AdamArgs a, const float4* __re
   }
   double s = block_sum(gn);
   if (threadIdx.x == 0 && partials) partials[blockIdx.x] = s;
-}
-
-// stats[0] = sum(loss partials) / n; stats[1] = sqrt(sum(grad-norm partials)).
-// One block of kStatsThreads; the loads are unrolled so that each thread has
-// its few partials in flight at once (a serial loop waited ~10 us on them).
-constexpr int kStatsThreads = 1024;
-__global__ void __launch_bounds__(kStatsThreads) k_finish_stats(const double* __restrict__ lp, int nl,
-                                                                const double* __restrict__ gp, int ng,
-                                                                const int* d_count, int n_max,
-                                                                double* __restrict__ stats) {
-  const int n = dev_count(d_count, n_max);
-  double a = 0.0, b = 0.0;
-#pragma unroll 4
-  for (int i = threadIdx.x; i < nl; i += kStatsThreads) a += lp[i];
-#pragma unroll 4
-  for (int i = threadIdx.x; i < ng; i += kStatsThreads) b += gp[i];
-  double sa = block_sum(a);
-  double sb = block_sum(b);
-  if (threadIdx.x == 0) {  // an empty batch ran no Adam pass: its gradient-norm partials are stale
-    stats[0] = n > 0 ? sa / double(n) : 0.0;
-    stats[1] = n > 0 ? sqrt(sb) : 0.0;
-  }
 }
 
 // Counter-based uniform in [0,1) for parameter initialisation (splitmix64).
@@ -304,10 +278,9 @@ nmg_status plain_pdf(nmg_ctx* c, const nmg_shading* in, const float* wi, const i
   return pdf_from_raw(c, w.raw, in, wi, d_count, n_max, pdf, st);
 }
 
-nmg_status optimizer_step(nmg_ctx* c, const int* d_count, int n_max, double* stats, cudaStream_t st) {
+nmg_status optimizer_step(nmg_ctx* c, const int* d_count, int n_max, int n_loss, double* stats, cudaStream_t st) {
   const Layout& L = c->lay;
   const nmg_config& g = c->cfg;
-  k_step_inc<<<1, 1, 0, st>>>(c->d_step, d_count);
   const int nb = 152 * 8;
   double* gp = c->ws.partials + c->ws.n_partials / 2;
   if (L.n_params % 4 || L.n_mlp % 4) return set_error(NMG_ERR_UNSUPPORTED, "parameter count not a multiple of 4");
@@ -338,12 +311,7 @@ nmg_status optimizer_step(nmg_ctx* c, const int* d_count, int n_max, double* sta
                                           reinterpret_cast<float4*>(c->v), reinterpret_cast<uint4*>(c->psteps),
                                           reinterpret_cast<float4*>(c->w_inf), nullptr, nullptr, gp, d_count);
   NMG_TRY(check_launch("k_adam_ema"));
-  if (stats) {
-    k_finish_stats<<<1, kStatsThreads, 0, st>>>(c->ws.partials, c->ws.n_partials / 2, gp, nb, d_count, n_max,
-                                                stats);
-    NMG_TRY(check_launch("k_finish_stats"));
-  }
-  return NMG_OK;
+  return finish_step(c, c->ws.partials, n_loss, gp, nb, d_count, n_max, stats, c->d_step, st);
 }
 
 nmg_status plain_train_step(nmg_ctx* c, const float* x, const float* rec, const int* d_count, int n_max,
@@ -353,7 +321,6 @@ nmg_status plain_train_step(nmg_ctx* c, const float* x, const float* rec, const 
   NMG_TRY(plain_forward(c, nullptr, x, d_count, n_max, c->w, true, w.raw, st));
   const int lb = blocks_for(n_max, 128, 4);
   if (lb > w.n_partials / 2) return set_error(NMG_ERR_CAPACITY, "loss partials");
-  cudaMemsetAsync(w.partials, 0, sizeof(double) * (w.n_partials / 2), st);
 #define LOSS(KK)                                                                                                  \
   if (c->cfg.selection)                                                                                           \
     k_train_loss<KK, true><<<lb, 128, 0, st>>>(w.raw, L.n_out_pad, rec, L.record_floats, c->mix, c->cfg.loss_scale, \
@@ -371,7 +338,7 @@ nmg_status plain_train_step(nmg_ctx* c, const float* x, const float* rec, const 
   NMG_TRY(check_launch("k_train_loss"));
   NMG_CUDA_TRY(cudaMemsetAsync(c->grad, 0, sizeof(float) * L.n_params, st));
   NMG_TRY(plain_backward(c, x, d_count, n_max, c->w, c->grad, st));
-  return optimizer_step(c, d_count, n_max, stats, st);
+  return optimizer_step(c, d_count, n_max, lb, stats, st);
 }
 
 // Network VJP at the training weights: draw given, accumulate unscaled
