@@ -18,6 +18,26 @@
 
 namespace nmg {
 
+// e^x = 2^(x log2 e) on the hardware's exponential and 1/x on its reciprocal,
+// both with subnormal results flushed to zero, which saves the instructions
+// that scale around them (__expf and __fdividef keep subnormals): for values
+// that cannot be subnormal, or whose subnormals round away in the sum that
+// follows. The results are then theirs, bit for bit.
+NMG_D float exp_ftz(float x) {
+  float r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x * 1.44269504f));
+  return r;
+}
+NMG_D float rsqrt_ftz(float x) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+NMG_D float rcp_ftz(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
 template <bool FAST> NMG_D float xexp(float x) { return FAST ? __expf(x) : expf(x); }
 template <bool FAST> NMG_D void xsincos(float x, float* s, float* c) {
   if (FAST)
@@ -286,7 +306,7 @@ NMG_D void lobe_angles(float st, float sp, float* sth, float* cth, float* sph, f
 // kernel: the extra live values made its consumer warps spill.)
 template <bool FAST> NMG_D float one_minus_exp_neg(float x) {
   if (!FAST) return -expm1f(-x);
-  if (x >= 0.5f) return 1.f - __expf(-x);
+  if (x >= 0.5f) return 1.f - exp_ftz(-x);
   return x * (1.f - x * (1.f / 2.f) * (1.f - x * (1.f / 3.f) * (1.f - x * (1.f / 4.f) *
              (1.f - x * (1.f / 5.f) * (1.f - x * (1.f / 6.f) * (1.f - x * (1.f / 7.f)))))));
 }
@@ -295,7 +315,7 @@ template <bool FAST> NMG_D float one_minus_exp_neg(float x) {
 NMG_D float one_minus_exp_neg_flat(float x) {
   const float lo = x * (1.f - x * (1.f / 2.f) * (1.f - x * (1.f / 3.f) * (1.f - x * (1.f / 4.f) *
                    (1.f - x * (1.f / 5.f) * (1.f - x * (1.f / 6.f) * (1.f - x * (1.f / 7.f)))))));
-  const float hi = 1.f - __expf(-x);
+  const float hi = 1.f - exp_ftz(-x);
   return x >= 0.5f ? hi : lo;
 }
 template <bool FAST> NMG_D f3 unit3(f3 a) {
@@ -308,7 +328,11 @@ template <bool FAST> NMG_D f3 unit3(f3 a) {
 
 // train.h:391-415 activations.
 NMG_D float act_exp_clamp(float x) { return fminf(fmaxf(x, -10.f), 15.f); }
-template <bool FAST> NMG_D float logistic(float x) { return xdiv<FAST>(1.f, 1.f + xexp<FAST>(-x)); }
+// e^x for x in the clamped range.
+template <bool FAST> NMG_D float act_exp(float x) { return FAST ? exp_ftz(act_exp_clamp(x)) : expf(act_exp_clamp(x)); }
+template <bool FAST> NMG_D float logistic(float x) {
+  return FAST ? rcp_ftz(1.f + exp_ftz(-x)) : 1.f / (1.f + expf(-x));
+}
 // Softplus in the stable form max(x,0) + log1p(e^-|x|) (train.h:398 writes
 // log(1+e^x), which loses all digits for x < -16).
 template <bool FAST> NMG_D float softplus(float x) {
@@ -341,7 +365,7 @@ template <bool FAST> NMG_D float vmf_norm(float k) {
 
 // vmf_norm<true> and (below) prod_norm<true> without branches.
 NMG_D float vmf_norm_flat(float k) {
-  const float v = __fdividef(k, NMG_TWO_PI * one_minus_exp_neg_flat(2.f * k));
+  const float v = k * rcp_ftz(NMG_TWO_PI * one_minus_exp_neg_flat(2.f * k));
   return k < NMG_EPS ? NMG_INV_4PI : v;
 }
 
@@ -353,8 +377,8 @@ NMG_D void mix_activate(Mix<K>& m, const float* raw, int kappa_softplus) {
 #pragma unroll
   for (int i = 0; i < K; ++i) {
     float4 r = reinterpret_cast<const float4*>(raw)[i];
-    m.lam[i] = xexp<FAST>(act_exp_clamp(r.x));
-    m.kap[i] = kappa_softplus ? softplus<FAST>(r.y) : xexp<FAST>(act_exp_clamp(r.y));
+    m.lam[i] = act_exp<FAST>(r.x);
+    m.kap[i] = kappa_softplus ? softplus<FAST>(r.y) : act_exp<FAST>(r.y);
     float st, ct, sp, cp;
     lobe_angles<FAST, PRECISE>(logistic<FAST>(r.z), logistic<FAST>(r.w), &st, &ct, &sp, &cp);
     m.mu[i] = f3{st * cp, st * sp, ct};
@@ -372,8 +396,8 @@ NMG_D void mix_activate(Mix<K>& m, const float* raw, int kappa_softplus) {
 template <bool FAST>
 NMG_D void lobe_activate(float r0, float r1, float r2, float r3, int kappa_softplus, float& lam, float& kap,
                          f3& mu) {
-  lam = xexp<FAST>(act_exp_clamp(r0));
-  kap = kappa_softplus ? softplus<FAST>(r1) : xexp<FAST>(act_exp_clamp(r1));
+  lam = act_exp<FAST>(r0);
+  kap = kappa_softplus ? softplus<FAST>(r1) : act_exp<FAST>(r1);
   float st, ct, sp, cp;
   lobe_angles<FAST, !FAST>(logistic<FAST>(r2), logistic<FAST>(r3), &st, &ct, &sp, &cp);
   mu = f3{st * cp, st * sp, ct};
@@ -404,7 +428,7 @@ template <bool FAST> NMG_D float prod_norm(float k) {
   return k < 1e-3f ? NMG_INV_4PI : xdiv<FAST>(k * NMG_INV_2PI, one_minus_exp_neg<FAST>(2.f * k));
 }
 NMG_D float prod_norm_flat(float k) {
-  const float v = __fdividef(k * NMG_INV_2PI, one_minus_exp_neg_flat(2.f * k));
+  const float v = k * NMG_INV_2PI * rcp_ftz(one_minus_exp_neg_flat(2.f * k));
   return k < 1e-3f ? NMG_INV_4PI : v;
 }
 constexpr float kCosineKappa = 2.18853f;  // distribution.h:184-195
@@ -422,7 +446,7 @@ NMG_D void lobe_cosine_flat(f3 mb, float nb, float& lam, float& kap, f3& mu, flo
   f3 nm = LOBE_FIRST ? f3{fmaf(ma.x, ka, mb.x * kb), fmaf(ma.y, ka, mb.y * kb), fmaf(ma.z, ka, mb.z * kb)}
                      : f3{fmaf(mb.x, kb, ma.x * ka), fmaf(mb.y, kb, ma.y * ka), fmaf(mb.z, kb, ma.z * ka)};
   const float n2 = dot3(nm, nm);
-  const float rn = rsqrtf(n2);
+  const float rn = rsqrt_ftz(n2);
   float nk = n2 * rn;
   const bool some = nk >= 1e-3f;
   nm = f3{some ? nm.x * rn : ma.x, some ? nm.y * rn : ma.y, some ? nm.z * rn : ma.z};
@@ -430,7 +454,7 @@ NMG_D void lobe_cosine_flat(f3 mb, float nb, float& lam, float& kap, f3& mu, flo
   const float e = __expf(ka * (dot3(nm, ma) - 1.f) + kb * (dot3(nm, mb) - 1.f));
   const float pk = prod_norm_flat(nk);
   const float pa = ka < 1e-3f ? NMG_INV_4PI : nrm;
-  lam = __fdividef(pa * nb, pk) * e * lam;
+  lam = pa * nb * rcp_ftz(pk) * e * lam;
   kap = nk;
   mu = nm;
   nrm = pk;
@@ -618,7 +642,7 @@ NMG_HD float bernoulli_gen(float x) {
 NMG_D float vmf_norm_sel(float k) {
   const float x = 2.f * k;
   const float lo = NMG_INV_4PI * bernoulli_gen(x);
-  const float hi = __fdividef(k * NMG_INV_2PI, 1.f - __expf(-x));
+  const float hi = k * NMG_INV_2PI * rcp_ftz(1.f - exp_ftz(-x));
   return x < 0.5f ? lo : hi;
 }
 
@@ -657,8 +681,8 @@ NMG_D void mix_activate_lean(MixLean<K>& m, const float* raw, int kappa_softplus
 #pragma unroll
   for (int i = 0; i < K; ++i) {
     const float4 r = WIDE ? row[WIDE ? i : 0] : reinterpret_cast<const float4*>(raw)[i];
-    m.lam[i] = __expf(act_exp_clamp(r.x));
-    float k = kappa_softplus ? softplus<true>(r.y) : __expf(act_exp_clamp(r.y));
+    m.lam[i] = act_exp<true>(r.x);
+    float k = kappa_softplus ? softplus<true>(r.y) : act_exp<true>(r.y);
     k = k < NMG_EPS ? 0.f : k;
     m.kap[i] = k;
     float st, ct, sp, cp;
@@ -702,6 +726,41 @@ NMG_D float mix_pdf_lean_sum(const MixLean<K>& m, f3 wi) {
 #pragma unroll
   for (int i = 0; i < K; ++i) p = fmaf(m.ln[i], __expf(m.kap[i] * fminf(0.f, dot3(wi, m.mu[i]) - 1.f)), p);
   return p;
+}
+
+// One lobe's share of the mixture pdf at wi (unit) from its raw outputs r: adds
+// the lobe's lambda to *total and lambda * vMF(wi) to *p, so that the pdf is
+// p / total and no lobe is kept. COS: of the lobe's product with the cosine lobe
+// around the unit vector mb (distribution.h:39-64, nb its normaliser): with the
+// product's normaliser pk, its lambda is a / pk and lambda * vMF a e^{..}. The
+// fused multiply-adds are stated: kappa up to 1000 and more turns a mean that
+// is rounded another way into 1e-4 of the pdf.
+NMG_D float dot3_fma(f3 a, f3 b) { return fmaf(a.x, b.x, fmaf(a.y, b.y, a.z * b.z)); }
+template <bool COS>
+NMG_D void lobe_pdf_lean(float4 r, int kappa_softplus, f3 wi, f3 mb, float nb, float* total, float* p) {
+  const float lam = act_exp<true>(r.x);
+  const float ka = kappa_softplus ? softplus<true>(r.y) : act_exp<true>(r.y);
+  float st, ct, sp, cp;
+  lobe_angles<true, kAngTab>(logistic<true>(r.z), logistic<true>(r.w), &st, &ct, &sp, &cp);
+  const f3 ma{st * cp, st * sp, ct};
+  if (!COS) {
+    const float k = ka < NMG_EPS ? 0.f : ka;
+    *total += lam;
+    *p = fmaf(lam * vmf_norm_sel(k), __expf(k * fminf(0.f, dot3(wi, ma) - 1.f)), *p);
+    return;
+  }
+  const float kb = kCosineKappa;
+  f3 nm{fmaf(ma.x, ka, mb.x * kb), fmaf(ma.y, ka, mb.y * kb), fmaf(ma.z, ka, mb.z * kb)};
+  const float n2 = dot3_fma(nm, nm), rn = rsqrt_ftz(n2);
+  const bool some = n2 * rn >= 1e-3f;
+  const float nk = some ? n2 * rn : 0.f;
+  nm = f3{some ? nm.x * rn : ma.x, some ? nm.y * rn : ma.y, some ? nm.z * rn : ma.z};
+  const float e = __expf(fmaf(ka, dot3_fma(nm, ma) - 1.f, kb * (dot3_fma(nm, mb) - 1.f)));
+  const float a = (ka < 1e-3f ? NMG_INV_4PI : vmf_norm_sel(ka)) * nb * e * lam;
+  const float x = 2.f * nk;  // 1 / pk: 4 pi / B(x), or 2 pi (1 - e^{-x}) / nk where that does not cancel
+  const bool lo = x < 0.5f;
+  *total = fmaf(a, (lo ? 4.f * NMG_PI : NMG_TWO_PI * (1.f - exp_ftz(-x))) * rcp_ftz(lo ? bernoulli_gen(x) : nk), *total);
+  *p = fmaf(a, __expf(nk * fminf(0.f, dot3_fma(wi, nm) - 1.f)), *p);
 }
 
 // vmf.h:48-71 for one lobe (kappa k, 0 for uniform; unit mean mu) with one
@@ -757,12 +816,12 @@ NMG_D float mix_kl_loss_grad(const RAW& raw, const float* rec, float scale, cons
 #pragma unroll
   for (int i = 0; i < K; ++i) {
     float4 r = lobe4(raw, i);
-    lam[i] = xexp<FAST>(act_exp_clamp(r.x));
+    lam[i] = act_exp<FAST>(r.x);
     if (o.kappa_softplus) {
       kap[i] = softplus<FAST>(r.y);
       dkap[i] = logistic<FAST>(r.y);
     } else {
-      kap[i] = xexp<FAST>(act_exp_clamp(r.y));
+      kap[i] = act_exp<FAST>(r.y);
       dkap[i] = kap[i];  // train.h:410: derivative ignores the clamp
     }
     sgt[i] = logistic<FAST>(r.z);
@@ -834,12 +893,12 @@ NMG_D float mix_kl_loss_grad_selection(const RAW& raw, const float* rec, float s
 #pragma unroll
   for (int i = 0; i < K; ++i) {
     float4 r = lobe4(raw, i);
-    lam[i] = xexp<FAST>(act_exp_clamp(r.x));
+    lam[i] = act_exp<FAST>(r.x);
     if (o.kappa_softplus) {
       kap[i] = softplus<FAST>(r.y);
       dkap[i] = logistic<FAST>(r.y);
     } else {
-      kap[i] = xexp<FAST>(act_exp_clamp(r.y));
+      kap[i] = act_exp<FAST>(r.y);
       dkap[i] = kap[i];
     }
     sgt[i] = logistic<FAST>(r.z);
@@ -924,13 +983,13 @@ NMG_D void half_loss_lobes(HalfLoss<KH>& s, const RAW& raw, const float* rec, co
 #pragma unroll
   for (int i = 0; i < KH; ++i) {
     const float4 r = lobe4(raw, i);
-    const float lam = xexp<FAST>(act_exp_clamp(r.x));
+    const float lam = act_exp<FAST>(r.x);
     float kap, dkap;
     if (o.kappa_softplus) {
       kap = softplus<FAST>(r.y);
       dkap = logistic<FAST>(r.y);
     } else {
-      kap = xexp<FAST>(act_exp_clamp(r.y));
+      kap = act_exp<FAST>(r.y);
       dkap = kap;  // train.h:410: derivative ignores the clamp
     }
     const float sgt = logistic<FAST>(r.z), sgp = logistic<FAST>(r.w);
@@ -944,7 +1003,7 @@ NMG_D void half_loss_lobes(HalfLoss<KH>& s, const RAW& raw, const float* rec, co
       // the normaliser and of d log(normaliser) / d kappa evaluated and one selected
       const float kz = k < NMG_EPS ? 0.f : k;
       vmf = __expf(kz * fminf(0.f, cc - 1.f)) * vmf_norm_sel(kz);
-      const float e = __expf(-2.f * k);
+      const float e = exp_ftz(-2.f * k);
       const float ik_exact = 1.f / k - (1.f + e) / (1.f - e);
       const float ik_small = o.kappa_poly ? 0.000926f + -0.344883f * k + 0.030147f * (k * k)
                                           : k * (-1.f / 3.f + k * k * (1.f / 45.f));

@@ -1,9 +1,9 @@
 // mixture_kernels.cu -- FP32 mixture kernels on raw network outputs and their
 // C-ABI entry points (nmg_mixture_*).
 //
-// Sampling takes one thread per query, the pdf and the loss a lane pair per
-// query (half the lobes each); lobes in registers; grid-stride loops over one
-// wave of resident blocks. Each query reads its raw row directly: 32-byte
+// Sampling takes one thread per query, and so does the pdf with the cosine lobe
+// or of odd K; the other pdfs and the loss take a lane pair per query (half the
+// lobes each); grid-stride loops over one wave of resident blocks. Each query reads its raw row directly: 32-byte
 // loads (two lobes) where the rows are 32-byte aligned for sampling and the
 // loss, else 16-byte loads (one lobe); its uniforms as one float4.
 #include <stdarg.h>
@@ -91,7 +91,8 @@ NMG_D void sample_one(const float* row, float4 u, const float* cosn, long q, int
 // 98 us with 16-byte loads (the L1 data pipe was then 73% busy with their
 // wavefronts, one line per lane and load), 115 us with the rows staged in
 // shared memory by per-thread cp.async copies (6 blocks per SM at 80
-// registers), 108 us with 106 registers and 4 blocks.
+// registers), 108 us with 106 registers and 4 blocks. Since then 88 -> 80 us
+// with exp_ftz and rcp_ftz (instruction issue was 61-69% busy).
 template <int K, bool FAST, bool COS, bool WIDE = false>
 __global__ void __launch_bounds__(kThreads, K <= 8 ? 5 : 1) k_mixture_sample(const float* __restrict__ raw,
                                                                              int stride,
@@ -112,20 +113,6 @@ __global__ void __launch_bounds__(kThreads, K <= 8 ? 5 : 1) k_mixture_sample(con
 // multiple of 8 floats from a 32-byte aligned base.
 static bool rows_32b(const float* raw, int stride) {
   return stride % 8 == 0 && (reinterpret_cast<uintptr_t>(raw) & 31u) == 0;
-}
-
-template <int K, bool FAST>
-__global__ void __launch_bounds__(kThreads) k_mixture_pdf(const float* __restrict__ raw, int stride,
-                                                          const float* __restrict__ wi,
-                                                          const float* __restrict__ cosn, int n,
-                                                          int kappa_softplus, float* __restrict__ pdf) {
-  sincospi_tab_fill();
-  for (long q = long(blockIdx.x) * blockDim.x + threadIdx.x; q < n; q += long(gridDim.x) * blockDim.x) {
-    Mix<K> m;
-    mix_activate<K, FAST, kAngTab>(m, raw + q * stride, kappa_softplus);
-    if (cosn) mix_apply_cosine<K, FAST>(m, load3(cosn, q));
-    pdf[q] = mix_pdf<K, FAST>(m, load3(wi, q));
-  }
 }
 
 // Sums `v` over the block in a fixed order; the result is valid in thread 0.
@@ -187,41 +174,14 @@ __global__ void k_sum_partials(const double* __restrict__ partials, int m, doubl
 NMG_D unsigned pair_mask() { return 3u << ((threadIdx.x & 31) & ~1u); }
 NMG_D float pair_sum(float v) { return v + __shfl_xor_sync(pair_mask(), v, 1); }
 
-// Weights from the pair's total (after activation or the cosine product).
-template <int KH, bool FAST>
-NMG_D void pair_weights(Mix<KH>& m, float total) {
-  m.total = total;
-  const float inv = 1.f / total;
-#pragma unroll
-  for (int i = 0; i < KH; ++i) m.w[i] = FAST ? m.lam[i] * inv : m.lam[i] / total;
-}
-
-template <int K, bool FAST>
-NMG_D void pair_mixture(Mix<K / 2>& m, const float* half_row, const float* cosn, long q, int kappa_softplus) {
-  constexpr int KH = K / 2;
-  mix_activate<KH, FAST, kAngTab>(m, half_row, kappa_softplus);
-  float lt = 0.f;
-#pragma unroll
-  for (int i = 0; i < KH; ++i) lt += m.lam[i];
-  pair_weights<KH, FAST>(m, pair_sum(lt));
-  if (cosn) {
-    mix_apply_cosine<KH, FAST>(m, load3(cosn, q));
-    lt = 0.f;
-#pragma unroll
-    for (int i = 0; i < KH; ++i) lt += m.lam[i];
-    pair_weights<KH, FAST>(m, fmaxf(pair_sum(lt), NMG_EPS));  // distribution.h:191
-  }
-}
-
-// Direct loads, one wave of resident blocks. COS: with the cosine-lobe
-// product; without it each lane sums lambda * vMF of its lobes in the lean
-// form and the pdf is the pair's sum over the pair's total. 8 blocks per SM
-// at K <= 8 (56 registers): 70 us for 2,097,152 queries at K = 8, against
-// 80 us with the rows staged in shared memory by per-thread cp.async copies.
-template <int K, bool FAST, bool COS>
+// The pdf of even K without the cosine lobe: direct loads, one wave of resident
+// blocks, each lane sums lambda * vMF of its lobes in the lean form and the pdf
+// is the pair's sum over the pair's total. 8 blocks per SM at K <= 8 (56
+// registers): 70 us for 2,097,152 queries at K = 8, against 80 us with the rows
+// staged in shared memory by per-thread cp.async copies.
+template <int K>
 __global__ void __launch_bounds__(kThreads, K <= 8 ? 8 : 1) k_mixture_pdf2(const float* __restrict__ raw, int stride,
-                                                                         const float* __restrict__ wi,
-                                                                         const float* __restrict__ cosn, int n,
+                                                                         const float* __restrict__ wi, int n,
                                                                          int kappa_softplus, float* __restrict__ pdf) {
   constexpr int KH = K / 2;
   const int h = threadIdx.x & 1;
@@ -231,17 +191,34 @@ __global__ void __launch_bounds__(kThreads, K <= 8 ? 8 : 1) k_mixture_pdf2(const
     const long q = t >> 1;
     const float* half_row = raw + q * stride + h * KH * 4;
     const f3 w = load3(wi, q);
-    float p;
-    if constexpr (FAST && !COS) {
-      MixLean<KH> m;
-      mix_activate_lean<KH>(m, half_row, kappa_softplus);
-      p = pair_sum(mix_pdf_lean_sum<KH>(m, w)) / pair_sum(m.total);
-    } else {
-      Mix<KH> m;
-      pair_mixture<K, FAST>(m, half_row, cosn, q, kappa_softplus);
-      p = pair_sum(mix_pdf<KH, FAST>(m, w));
-    }
+    MixLean<KH> m;
+    mix_activate_lean<KH>(m, half_row, kappa_softplus);
+    const float p = pair_sum(mix_pdf_lean_sum<KH>(m, w)) / pair_sum(m.total);
     if (h == 0) pdf[q] = p;
+  }
+}
+
+// The other pdfs (with the cosine lobe, or odd K): one thread per query sums
+// its lobes one after the other and keeps none, so that 8 blocks fit an SM.
+// Instruction issue and the special-function unit bound it. 300,001 queries at
+// K = 7 with the cosine lobe: 16.0 us (two lanes per query 18.9, four 20.9;
+// the lobes kept and the product's branches taken 25.6); 2,000,000 at K = 8:
+// 83 us (a lane pair with its lobes kept 127).
+template <int K, bool COS>
+__global__ void __launch_bounds__(kThreads, 8) k_mixture_pdf(const float* __restrict__ raw, int stride,
+                                                             const float* __restrict__ wi,
+                                                             const float* __restrict__ cosn, int n,
+                                                             int kappa_softplus, float* __restrict__ pdf) {
+  sincospi_tab_fill();
+  const float nb = prod_norm<true>(kCosineKappa);
+  const long step = long(gridDim.x) * blockDim.x;
+  for (long q = long(blockIdx.x) * blockDim.x + threadIdx.x; q < n; q += step) {
+    const float4* row = reinterpret_cast<const float4*>(raw + q * stride);
+    const f3 w = load3(wi, q), mb = COS ? unit3<true>(load3(cosn, q)) : f3{0.f, 0.f, 1.f};
+    float total = 0.f, p = 0.f;
+#pragma unroll
+    for (int i = 0; i < K; ++i) lobe_pdf_lean<COS>(row[i], kappa_softplus, w, mb, nb, &total, &p);
+    pdf[q] = p / (COS ? fmaxf(total, NMG_EPS) : total);  // distribution.h:191
   }
 }
 
@@ -286,12 +263,12 @@ __global__ void __launch_bounds__(kThreads, K <= 8 ? 8 : 1) k_mixture_loss_grad2
 #pragma unroll
     for (int i = 0; i < KH; ++i) {
       const float4 x = WIDE ? xw[WIDE ? i : 0] : reinterpret_cast<const float4*>(row)[i];
-      lam[i] = xexp<FAST>(act_exp_clamp(x.x));
+      lam[i] = act_exp<FAST>(x.x);
       if (o.kappa_softplus) {
         kap[i] = softplus<FAST>(x.y);
         dkap[i] = logistic<FAST>(x.y);
       } else {
-        kap[i] = xexp<FAST>(act_exp_clamp(x.y));
+        kap[i] = act_exp<FAST>(x.y);
         dkap[i] = kap[i];  // train.h:410: the derivative ignores the clamp
       }
       sgt[i] = logistic<FAST>(x.z);
@@ -329,7 +306,7 @@ __global__ void __launch_bounds__(kThreads, K <= 8 ? 8 : 1) k_mixture_loss_grad2
       const float wv = (lam[i] * inv_total) * vmf[i];
       // d log(vMF normaliser) / d kappa (distribution.h:160-172): the polynomial below kappa 1 or the
       // series below 1e-2, else 1/k - coth(k); both forms evaluated and one selected (no divergence)
-      const float e = xexp<FAST>(-2.f * k);
+      const float e = exp_ftz(-2.f * k);
       const float ik_exact = xdiv<FAST>(1.f, k) - xdiv<FAST>(1.f + e, 1.f - e);
       const float ik_small = o.kappa_poly ? 0.000926f + -0.344883f * k + 0.030147f * (k * k)
                                           : k * (-1.f / 3.f + k * k * (1.f / 45.f));
@@ -380,20 +357,17 @@ static nmg_status launch_sample(const nmg_mixture_opts* o, const float* raw, con
 template <int K>
 static nmg_status launch_pdf(const nmg_mixture_opts* o, const float* raw, const float* wi, const float* cosn, int n,
                              float* pdf, cudaStream_t st) {
-  if constexpr (K % 2 == 0) {
-    if (cosn) {
-      const int grid = resident_grid(k_mixture_pdf2<K, kMixFast, true>, 0, 2L * n);
-      k_mixture_pdf2<K, kMixFast, true><<<grid, kThreads, 0, st>>>(raw, o->stride, wi, cosn, n, o->kappa_softplus,
-                                                                   pdf);
-    } else {
-      // (the 32-byte row loads of the sampler and the loss measured 71.7 against 69.6 us here)
-      const int grid = resident_grid(k_mixture_pdf2<K, kMixFast, false>, 0, 2L * n);
-      k_mixture_pdf2<K, kMixFast, false><<<grid, kThreads, 0, st>>>(raw, o->stride, wi, nullptr, n,
-                                                                    o->kappa_softplus, pdf);
-    }
+  if (cosn) {
+    const int grid = resident_grid(k_mixture_pdf<K, true>, 0, n);
+    k_mixture_pdf<K, true><<<grid, kThreads, 0, st>>>(raw, o->stride, wi, cosn, n, o->kappa_softplus, pdf);
+  } else if constexpr (K % 2 == 0) {
+    // (the 32-byte row loads of the sampler and the loss measured 71.7 against 69.6 us here)
+    const int grid = resident_grid(k_mixture_pdf2<K>, 0, 2L * n);
+    k_mixture_pdf2<K><<<grid, kThreads, 0, st>>>(raw, o->stride, wi, n, o->kappa_softplus, pdf);
+  } else {
+    const int grid = resident_grid(k_mixture_pdf<K, false>, 0, n);
+    k_mixture_pdf<K, false><<<grid, kThreads, 0, st>>>(raw, o->stride, wi, cosn, n, o->kappa_softplus, pdf);
   }
-  else
-    k_mixture_pdf<K, kMixFast><<<grid_for(n), kThreads, 0, st>>>(raw, o->stride, wi, cosn, n, o->kappa_softplus, pdf);
   return check_launch("nmg_mixture_pdf");
 }
 
