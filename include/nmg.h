@@ -109,7 +109,11 @@ nmg_status nmg_mixture_loss_grad(const nmg_mixture_opts* opts, const float* raw,
                                  int record_stride, int n, float loss_scale, float* grad, float* loss,
                                  double* loss_sum, void* workspace, size_t workspace_bytes,
                                  nmg_stream stream);
-
+/* The same, with the padding columns of grad set to 0 by the same kernel. */
+nmg_status nmg_mixture_loss_grad_rows(const nmg_mixture_opts* opts, const float* raw, const float* record,
+                                      int record_stride, int n, float loss_scale, float* grad, float* loss,
+                                      double* loss_sum, void* workspace, size_t workspace_bytes,
+                                      nmg_stream stream);
 
 /*
  * nmg_mixture_loss_grad without a caller-provided workspace. This entry point

@@ -55,7 +55,8 @@ def lib():
         L.nmg_mixture_loss_workspace_bytes.argtypes = [C.c_int]
         L.nmg_mixture_loss_grad.argtypes = [C.POINTER(MixtureOpts), P, P, C.c_int, C.c_int, C.c_float, P, P, P, P,
                                             C.c_size_t, P]
-        for name in ("nmg_mixture_sample", "nmg_mixture_pdf", "nmg_mixture_loss_grad"):
+        L.nmg_mixture_loss_grad_rows.argtypes = L.nmg_mixture_loss_grad.argtypes
+        for name in ("nmg_mixture_sample", "nmg_mixture_pdf", "nmg_mixture_loss_grad", "nmg_mixture_loss_grad_rows"):
             getattr(L, name).restype = C.c_int
         _lib = L
     return _lib
@@ -110,15 +111,15 @@ def mixture_loss_grad(raw, records, n_lobes, loss_scale=128.0, selection=False, 
     import torch
     n = raw.shape[0]
     dev = raw.device
-    g = torch.zeros_like(raw)
+    g = torch.empty_like(raw)
     loss = torch.empty(n, device=dev, dtype=torch.float32) if want_loss else None
     tot = torch.empty(1, device=dev, dtype=torch.float64)
     L = lib()
     wsb = L.nmg_mixture_loss_workspace_bytes(n)
     ws = torch.empty(wsb, device=dev, dtype=torch.uint8)
     o = mixture_opts(n_lobes, raw.shape[1], kappa_softplus, kappa_poly, selection)
-    check(L.nmg_mixture_loss_grad(C.byref(o), _ptr(raw), _ptr(records), records.shape[1], n, float(loss_scale),
-                                  _ptr(g), _ptr(loss), _ptr(tot), _ptr(ws), wsb, _stream(stream)))
+    check(L.nmg_mixture_loss_grad_rows(C.byref(o), _ptr(raw), _ptr(records), records.shape[1], n, float(loss_scale),
+                                       _ptr(g), _ptr(loss), _ptr(tot), _ptr(ws), wsb, _stream(stream)))
     return g, loss, tot
 
 

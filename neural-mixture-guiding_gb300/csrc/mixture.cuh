@@ -343,6 +343,7 @@ struct MixOpts {
   int kappa_softplus;  // 0: kappa = exp(clamp(x)) (train.h:244); 1: log(1+e^x)
   int kappa_poly;      // 1: distribution.h:165-166 polynomial for kappa < 1
   int cosine;          // multiply by the cosine lobe before sampling/pdf
+  int zero_to;         // loss kernels: gradient columns from the outputs to this one are set to 0 (0: untouched)
 };
 
 template <int K> struct Mix {
