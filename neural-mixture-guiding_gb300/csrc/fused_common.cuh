@@ -562,6 +562,23 @@ NMG_D void encode_row_half(const FusedArgs& a, const float (&x)[10], uint8_t* ti
   static_assert(NGRID % 16 == 0, "grid chunks split evenly over the two halves");
   const bool fp16 = layer_fp16(a, 0);
   const float p3[3] = {x[0], x[1], x[2]};
+  float d[NPAD - NGRID];
+#pragma unroll
+  for (int k = 0; k < NPAD - NGRID; ++k) d[k] = 1.f;
+  if (MODE == 0) {
+    sh_basis(SHDEG, x[3] * 2.f - 1.f, x[4] * 2.f - 1.f, x[5] * 2.f - 1.f, d);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) oneblob_fixed<BINS>(x[6 + k], d + SHDEG * SHDEG + k * BINS);
+  } else if (!SPLIT_SH || h == 0) {
+    sh_basis(SHDEG, x[3] * 2.f - 1.f, x[4] * 2.f - 1.f, x[5] * 2.f - 1.f, d);
+  }
+  if (MODE == 1 && (!SPLIT_SH || h == 1)) {
+    sh_basis(SHDEG, x[6] * 2.f - 1.f, x[7] * 2.f - 1.f, x[8] * 2.f - 1.f, d + SHDEG * SHDEG);
+    oneblob_fixed<BINS>(x[9], d + 2 * SHDEG * SHDEG);
+  }
+#pragma unroll
+  for (int ch = 0; ch < DCH; ++ch)
+    if ((ch < DCH0) == (h == 0)) store_chunk(tile, row, GCH + ch, KC, d + 8 * ch, fp16);
   if constexpr (F == 2 && PAIR) {
     const bool out16 = fp16;
     const int l1 = h ? LEVELS : a.half_levels;
@@ -582,23 +599,6 @@ NMG_D void encode_row_half(const FusedArgs& a, const float (&x)[10], uint8_t* ti
       store_chunk(tile, row, ch, KC, f, fp16);
     }
   }
-  float d[NPAD - NGRID];
-#pragma unroll
-  for (int k = 0; k < NPAD - NGRID; ++k) d[k] = 1.f;
-  if (MODE == 0) {
-    sh_basis(SHDEG, x[3] * 2.f - 1.f, x[4] * 2.f - 1.f, x[5] * 2.f - 1.f, d);
-#pragma unroll
-    for (int k = 0; k < 3; ++k) oneblob_fixed<BINS>(x[6 + k], d + SHDEG * SHDEG + k * BINS);
-  } else if (!SPLIT_SH || h == 0) {
-    sh_basis(SHDEG, x[3] * 2.f - 1.f, x[4] * 2.f - 1.f, x[5] * 2.f - 1.f, d);
-  }
-  if (MODE == 1 && (!SPLIT_SH || h == 1)) {
-    sh_basis(SHDEG, x[6] * 2.f - 1.f, x[7] * 2.f - 1.f, x[8] * 2.f - 1.f, d + SHDEG * SHDEG);
-    oneblob_fixed<BINS>(x[9], d + 2 * SHDEG * SHDEG);
-  }
-#pragma unroll
-  for (int ch = 0; ch < DCH; ++ch)
-    if ((ch < DCH0) == (h == 0)) store_chunk(tile, row, GCH + ch, KC, d + 8 * ch, fp16);
 }
 
 // Loads network input row q (n_input <= 10 floats) with compile-time indices.

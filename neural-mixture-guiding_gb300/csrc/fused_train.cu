@@ -177,6 +177,11 @@ NMG_D void scatter_level(const FusedArgs& a, float* gt, int lv, const float (&p3
 // Registers: the 768-thread block launches at 80 per thread and moves 32 of
 // them from each issuer/scatter thread to the compute threads.
 constexpr int kScatThreadsPerCta = 6 * kRows;
+// The issuer and scatter threads take theirs back only when the compute threads
+// have returned them (barrier kRegBar): those of a CTA without tiles could
+// otherwise take them before the compute threads' request, which would then
+// wait for ever.
+constexpr int kRegBar = 3;
 constexpr int kScatRegLaunch = 80, kScatRegCompute = 96, kScatRegScatter = 48;
 static_assert(4 * kRows * kScatRegCompute + 2 * kRows * kScatRegScatter == kScatThreadsPerCta * kScatRegLaunch,
               "register split must equal the launch allocation");
@@ -374,7 +379,10 @@ __global__ void __launch_bounds__(SCAT ? kScatThreadsPerCta : 2 * NWG * kRows + 
       }
     }
     __syncwarp();
-    if constexpr (SCAT) tc::reg_alloc<kScatRegLaunch>();
+    if constexpr (SCAT) {
+      tc::bar_sync(kRegBar, kScatThreadsPerCta);
+      tc::reg_alloc<kScatRegLaunch>();
+    }
   } else if (scatter) {
     // ------------------------------------------------------- scatter warps
     tc::reg_dealloc<kScatRegScatter>();
@@ -413,6 +421,8 @@ __global__ void __launch_bounds__(SCAT ? kScatThreadsPerCta : 2 * NWG * kRows + 
       }
       if (!any) break;
     }
+    __syncwarp();
+    tc::bar_sync(kRegBar, kScatThreadsPerCta);
     tc::reg_alloc<kScatRegLaunch>();
   } else {
     // ---------------------------------------- pipeline g, half h of every row
@@ -632,7 +642,11 @@ __global__ void __launch_bounds__(SCAT ? kScatThreadsPerCta : 2 * NWG * kRows + 
         }
       }
     }
-    if constexpr (SCAT) tc::reg_dealloc<kScatRegLaunch>();
+    if constexpr (SCAT) {
+      __syncwarp();
+      tc::reg_dealloc<kScatRegLaunch>();
+      tc::bar_arrive(kRegBar, kScatThreadsPerCta);
+    }
   }
 
   // ---- flush the CTA's weight gradients (M = 64 accumulators) to global

@@ -286,6 +286,7 @@ template <int N> NMG_D void reg_alloc() { asm volatile("setmaxnreg.inc.sync.alig
 
 // Named barrier over `count` threads (a warpgroup = 128).
 NMG_D void bar_sync(int id, int count) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory"); }
+NMG_D void bar_arrive(int id, int count) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(count) : "memory"); }
 
 // max(a,0), max(b,0) packed into one bf16x2 / f16x2 word in one instruction.
 NMG_D uint32_t pack2_relu(float a, float b, bool fp16) {
