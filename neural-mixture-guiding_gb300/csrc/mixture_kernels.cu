@@ -92,9 +92,10 @@ NMG_D void sample_one(const float* row, float4 u, const float* cosn, long q, int
 // wavefronts, one line per lane and load), 115 us with the rows staged in
 // shared memory by per-thread cp.async copies (6 blocks per SM at 80
 // registers), 108 us with 106 registers and 4 blocks. Since then 88 -> 80 us
-// with exp_ftz and rcp_ftz (instruction issue was 61-69% busy).
+// with exp_ftz and rcp_ftz (instruction issue was 61-69% busy), and 78 with the
+// 80 registers of 6 blocks per SM that they leave room for (7 blocks: 82 us).
 template <int K, bool FAST, bool COS, bool WIDE = false>
-__global__ void __launch_bounds__(kThreads, K <= 8 ? 5 : 1) k_mixture_sample(const float* __restrict__ raw,
+__global__ void __launch_bounds__(kThreads, K <= 8 ? 6 : 1) k_mixture_sample(const float* __restrict__ raw,
                                                                              int stride,
                                                                              const float* __restrict__ u4,
                                                                              const float* __restrict__ cosn, int n,
