@@ -29,6 +29,10 @@ nmg_status set_error(nmg_status st, const char* fmt, ...) {
 }
 
 constexpr int kThreads = 128;
+// The lane-pair loss: two threads a sample, and as many blocks as kThreads
+// samples each, which the workspace has partial sums for (blocks of kThreads
+// went over a small batch twice with half the GPU: 4,096 samples 10.4 us).
+constexpr int kLossThreads = 2 * kThreads;
 
 // Hardware transcendental approximations (__expf, __fdividef, __sincosf for
 // the sampled azimuth): the reference compiles all of its CUDA with
@@ -48,12 +52,12 @@ static int grid_for(long n) {
 // One wave of the blocks that fit on the device at once (the kernels loop
 // over the queries with a grid stride), or fewer for small n.
 template <class Kern>
-static int resident_grid(Kern kernel, int smem, long n) {
+static int resident_grid(Kern kernel, int smem, long n, int threads = kThreads) {
   int dev = 0, sms = 152, per_sm = 1;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kThreads, smem) != cudaSuccess || per_sm < 1)
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem) != cudaSuccess || per_sm < 1)
     per_sm = 1;
-  const long blocks = (n + kThreads - 1) / kThreads, cap = long(sms) * per_sm;
+  const long blocks = (n + threads - 1) / threads, cap = long(sms) * per_sm;
   return int(blocks < cap ? (blocks > 0 ? blocks : 1) : cap);
 }
 
@@ -240,14 +244,14 @@ __global__ void __launch_bounds__(kThreads, 8) k_mixture_pdf(const float* __rest
 // train.cu:69-172 with the lobes split over a lane pair: each lane computes
 // its lobes' activations, vMF values and gradients; q and the total come
 // from the pair's partial sums. Direct loads (WIDE: 32-byte loads of the
-// half row, rows_32b); 8 blocks per SM at K <= 8 (64 registers). 2,097,152
+// half row, rows_32b); 4 blocks per SM at K <= 8 (64 registers), 2 at K = 16. 2,097,152
 // queries at K = 8: 152 us with 32-byte loads, 154 us with 16-byte loads,
 // 178 us with the rows staged in shared memory by per-thread cp.async copies,
 // 166 us at the 89 registers the compiler picks unbounded.
 // With the flushing exponentials and reciprocals and without a fill of the
 // gradient before it, 2,000,000 queries: 129 us (172 before, the fill included).
 template <int K, bool SEL, bool WIDE = false>
-__global__ void __launch_bounds__(kThreads, K <= 8 ? 8 : 1) k_mixture_loss_grad2(const float* __restrict__ raw,
+__global__ void __launch_bounds__(kLossThreads, K <= 8 ? 4 : 2) k_mixture_loss_grad2(const float* __restrict__ raw,
                                                                                int stride,
                                                                                const float* __restrict__ rec,
                                                                                int rstride, int n, float scale,
@@ -398,17 +402,17 @@ static nmg_status launch_loss(const nmg_mixture_opts* o, const float* raw, const
   const float scale = loss_scale / float(n);
   if constexpr (K % 2 == 0) {
     if (o->selection) {
-      blocks = std::min(blocks, resident_grid(k_mixture_loss_grad2<K, true>, 0, 2L * n));
-      k_mixture_loss_grad2<K, true><<<blocks, kThreads, 0, st>>>(raw, o->stride, rec, rstride, n, scale, mo, grad,
+      blocks = std::min(blocks, resident_grid(k_mixture_loss_grad2<K, true>, 0, 2L * n, kLossThreads));
+      k_mixture_loss_grad2<K, true><<<blocks, kLossThreads, 0, st>>>(raw, o->stride, rec, rstride, n, scale, mo, grad,
                                                                  loss, loss_sum ? partials : nullptr);
     } else if ((K / 2) % 2 == 0 && rows_32b(raw, o->stride)) {
       constexpr bool W = (K / 2) % 2 == 0;
-      blocks = std::min(blocks, resident_grid(k_mixture_loss_grad2<K, false, W>, 0, 2L * n));
-      k_mixture_loss_grad2<K, false, W><<<blocks, kThreads, 0, st>>>(raw, o->stride, rec, rstride, n, scale, mo,
+      blocks = std::min(blocks, resident_grid(k_mixture_loss_grad2<K, false, W>, 0, 2L * n, kLossThreads));
+      k_mixture_loss_grad2<K, false, W><<<blocks, kLossThreads, 0, st>>>(raw, o->stride, rec, rstride, n, scale, mo,
                                                                      grad, loss, loss_sum ? partials : nullptr);
     } else {
-      blocks = std::min(blocks, resident_grid(k_mixture_loss_grad2<K, false>, 0, 2L * n));
-      k_mixture_loss_grad2<K, false><<<blocks, kThreads, 0, st>>>(raw, o->stride, rec, rstride, n, scale, mo, grad,
+      blocks = std::min(blocks, resident_grid(k_mixture_loss_grad2<K, false>, 0, 2L * n, kLossThreads));
+      k_mixture_loss_grad2<K, false><<<blocks, kLossThreads, 0, st>>>(raw, o->stride, rec, rstride, n, scale, mo, grad,
                                                                   loss, loss_sum ? partials : nullptr);
     }
   } else {
@@ -600,10 +604,10 @@ static nmg_status launch_loss_noalloc(const nmg_mixture_opts* o, const float* ra
   // the kernels of nmg_mixture_loss_grad, so that both entry points give the same gradients
   if constexpr (K % 2 == 0) {
     if (o->selection)
-      k_mixture_loss_grad2<K, true><<<blocks, kThreads, 0, st>>>(raw, o->stride, rec, rstride, n, scale, mo, grad,
+      k_mixture_loss_grad2<K, true><<<blocks, kLossThreads, 0, st>>>(raw, o->stride, rec, rstride, n, scale, mo, grad,
                                                                  loss, loss_sum ? partials : nullptr);
     else
-      k_mixture_loss_grad2<K, false><<<blocks, kThreads, 0, st>>>(raw, o->stride, rec, rstride, n, scale, mo, grad,
+      k_mixture_loss_grad2<K, false><<<blocks, kLossThreads, 0, st>>>(raw, o->stride, rec, rstride, n, scale, mo, grad,
                                                                   loss, loss_sum ? partials : nullptr);
   } else {
     if (o->selection)
