@@ -41,13 +41,13 @@ N_QUERIES = 1920 * 1080
 N_TRAIN = 1 << 18
 FLOP_PER_QUERY = 2 * (80 * 64 + 64 * 64 + 64 * 64 + 64 * 48)  # 32,768 executed (padded) MLP FLOP
 BYTES_PER_QUERY = 12 + 12 + 12 + 4 + 16 + 12 + 4 + 4 + 4      # pos, wo, n, rough, u4 in; dir, pdf, lobe, sel out
-# dram__bytes_read.sum + dram__bytes_write.sum of one k_fused_query_ws launch over the same
-# 2,073,600-query wavefront (ncu capture summarised in profiles/k_fused_query_ws_hashgrid_2073600.md)
-TRAFFIC_QUERY_BYTES = 141_316_608 + 35_742_464
+# dram__bytes_read.sum + dram__bytes_write.sum of one k_fused_query_roles launch over the same
+# 2,073,600-query wavefront (ncu capture summarised in profiles/k_fused_query_roles_hashgrid_2073600.md)
+TRAFFIC_QUERY_BYTES = 144_258_816 + 35_709_696
 # l1tex__m_xbar2l1tex_read_bytes.sum of the same capture: the hash-grid corner gathers reaching L2
 # (the 24 MB table stays in L2), in 32-byte sectors; about one sector request per cycle per SM is
 # the ceiling a gather-only kernel of the same 128 corners per query reaches
-L2_TO_L1_BYTES = 4.686e9
+L2_TO_L1_BYTES = 4.054e9
 
 
 # The hash-grid network (NMG_PRESET_HASHGRID) as the oracle describes it; the CPU legs build it from this
@@ -382,12 +382,12 @@ def run_ours(args):
                 "api": "nmg_query_host + nmg_train_step_host (pinned host memory; inputs copied in, results "
                        "written by the kernels through the host mapping)", "final_loss": e2e_loss},
         "gpu_launches": None,
-        "roofline": {"kernel": "k_fused_query_ws" if path != nmg.PATH_FP32 else "plain query kernels",
+        "roofline": {"kernel": "k_fused_query_roles" if path != nmg.PATH_FP32 else "plain query kernels",
                      "bound": "tensor", "achieved": tflops, "peak": bf16, "unit": "TFLOP/s",
                      "frac": tflops / bf16, "peak_source": src,
                      "traffic": TRAFFIC_QUERY_BYTES if path == nmg.PATH_BF16 else None,
                      "traffic_unit": "bytes per launch (ncu)",
-                     "limiter": "hash-grid gathers: ~70 L2 sector requests per query, L1->L2 request path 74% busy "
+                     "limiter": "hash-grid gathers: ~61 L2 sectors per query, L1->L2 request path 76% busy "
                                 "(ncu), not HBM or the tensor pipe",
                      "hbm_achieved_gbs": gbs, "hbm_frac": gbs / hbm,
                      "l2_sector_requests": l2_request_roofline(t_kernel, ours["clocks"]),
