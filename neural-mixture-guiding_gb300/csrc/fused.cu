@@ -625,7 +625,7 @@ static nmg_status launch_query_pair(const FusedArgs& a, cudaStream_t st) {
 // Default query tiling: the kernels that give the mixture warpgroups of its own
 // (fused_ws.cu). Three roles for the hash-grid networks: tiling 12 at 8 lobes,
 // 535 us for a 2,073,600-query wavefront (one warpgroup for MLP and mixture:
-// 624 us; one pipeline per warpgroup: 759 us), tiling 7 at 16 lobes, 330 us for
+// 624 us; one pipeline per warpgroup: 759 us), tiling 7 at 16 lobes, 318 us for
 // 900,000 queries (two threads per query: 464 us). Two roles for the reference
 // network, tiling 8, whose 8 levels gather in half the time: 110 us for the pdf
 // of 550,001 queries (three roles: 122 us, before 150 us).

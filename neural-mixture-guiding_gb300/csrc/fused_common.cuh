@@ -273,7 +273,7 @@ NMG_D void cell_features(const FusedArgs& a, int l, const uint32_t (&g)[3], cons
 // query kernels take 648 instead of 678 us (warp-specialised) and 797
 // instead of 834 us (one pipeline per warpgroup), the training step 0.492
 // instead of 0.499 ms.
-template <int F, bool SMOOTH, bool PAIR = false, bool CELLS = true>
+template <int F, bool SMOOTH, bool PAIR = false>
 NMG_D void grid_level(const FusedArgs& a, int l, const float (&p3)[3], float* out) {
   float w[3];
   uint32_t g[3];
@@ -289,7 +289,7 @@ NMG_D void grid_level(const FusedArgs& a, int l, const float (&p3)[3], float* ou
   const float wz[2] = {1.f - w[2], w[2]};
   const uint32_t T = a.lvl_T[l];
   const uint32_t base = a.enc.offset[l];
-  if (CELLS && ((a.lvl_rec >> l) & 1u)) {
+  if ((a.lvl_rec >> l) & 1u) {
     cell_features<F>(a, l, g, w, wxy, wz, out);
     return;
   }
@@ -487,10 +487,9 @@ NMG_D void encode_direction(const float (&x)[10], uint8_t* tile, int row, bool f
 
 // Encodes one input row x into `tile` row `row` (KC 16-byte chunks).
 // UNROLL = false keeps one copy of the chunk body (smaller code for kernels
-// whose instruction footprint matters more than the loop overhead). Levels
-// are gathered one at a time: computing the corners of 2 or 4 levels first
-// and issuing all their table loads back to back measured slower in both
-// fused kernels.
+// whose instruction footprint matters more than the loop overhead). With PAIR
+// and two features a level's loads run ahead of the last one's blend
+// (encode_levels2); the other forms gather one level at a time.
 template <int F, int LEVELS, int MODE, int SHDEG, int BINS, bool SMOOTH, bool UNROLL = true, bool PAIR = false>
 NMG_D void encode_row(const FusedArgs& a, const float (&x)[10], uint8_t* tile, int row) {
   constexpr int NDIR = MODE == 0 ? SHDEG * SHDEG + 3 * BINS : 2 * SHDEG * SHDEG + BINS;

@@ -418,7 +418,7 @@ NMG_D void store_raw16(const FusedArgs& a, long q, int c16, const float (&r)[16]
 // At 8 lobes two mixture warpgroups with a tile each keep up (88 registers hold
 // a thread's 8 lobes); at 16 lobes the mixture takes as long as the gathers,
 // and four warpgroups share a tile (two threads per query: 464 us for 900,000
-// queries, now 330 us).
+// queries, now 318 us).
 // SHARE, for launches of up to kShareTiles tiles per SM: every tile is encoded
 // by all the encoder warpgroups, a part of the levels each, so that the first
 // one is ready in a third of the time and the tiles follow one another. With
