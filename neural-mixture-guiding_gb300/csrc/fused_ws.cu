@@ -744,6 +744,11 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) k_fused_query_duo(const __gri
   uint32_t* tslot = reinterpret_cast<uint32_t*>(wbar + 1);
   const int wg = threadIdx.x / kRows, t = threadIdx.x % kRows;
 
+  // A CTA without tiles (a device count below n_max) leaves before it starts
+  // anything: the weights are waited for before a warpgroup's first tile, so
+  // nobody would wait for its copy, and a CTA must not exit with a copy into its
+  // shared memory in flight.
+  if (long(blockIdx.x) * kRows >= fused_count(a.d_count, a.n_max)) return;
   if (threadIdx.x == 0) {
     for (int i = 0; i < N; ++i) {
       tc::mbar_init(&done[i], 1);
@@ -757,20 +762,17 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) k_fused_query_duo(const __gri
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
-  const int n = fused_count(a.d_count, a.n_max);
-  const long ntiles = (long(n) + kRows - 1) / kRows;
-  // this CTA's tiles: blockIdx.x + j gridDim.x for j < nj; tile j is warpgroup j % N's
-  const int nj = long(blockIdx.x) < ntiles ? int((ntiles - 1 - long(blockIdx.x)) / long(gridDim.x)) + 1 : 0;
-  // The weights are waited for before a warpgroup's first tile: a CTA without
-  // tiles (a device count below n_max) copies none, as nobody would wait for
-  // them and a CTA must not exit with a copy into its shared memory in flight.
-  if (threadIdx.x == 0 && nj > 0) {
+  if (threadIdx.x == 0) {
     tc::mbar_arrive_expect_tx(wbar, a.w_bytes);
     for (uint32_t off = 0; off < a.w_bytes; off += 16384u) {
       const uint32_t nb = a.w_bytes - off < 16384u ? a.w_bytes - off : 16384u;
       tc::bulk_g2s(wsm + off, a.wimg + off, nb, wbar);
     }
   }
+  const int n = fused_count(a.d_count, a.n_max);
+  const long ntiles = (long(n) + kRows - 1) / kRows;
+  // this CTA's tiles: blockIdx.x + j gridDim.x for j < nj; tile j is warpgroup j % N's
+  const int nj = long(blockIdx.x) < ntiles ? int((ntiles - 1 - long(blockIdx.x)) / long(gridDim.x)) + 1 : 0;
   bool ok = true;
 
   if (wg < N) {
