@@ -38,8 +38,13 @@ namespace nmg {
 // STREAM: the mixture epilogue reads the raw outputs from TMEM lobe group by
 // lobe group (query_epilogue_streamed) instead of holding them in registers;
 // used for 16-lobe queries that return no raw outputs.
+// AHEAD: encode_row's. Where the registers are few (5 and 6 warpgroups) the
+// second level in flight spills; 500,000 queries of the hash-grid network with
+// and without: 5 warpgroups 260 and 217 us, 6 warpgroups 365 and 286 us; the
+// raw outputs alone at 16 lobes, 4 warpgroups, 247 and 221 us, but with the
+// mixture beside them 424 and 533 us.
 template <int F, int LEVELS, int MODE, int SHDEG, int BINS, int K, int NOUTMAX, bool SMOOTH, int NWG,
-          bool STREAM = false>
+          bool STREAM = false, bool AHEAD = NWG <= 4>
 __global__ void __launch_bounds__(NWG * kRows, 1) k_fused_query(const __grid_constant__ FusedArgs a) {
   constexpr int NDIR = MODE == 0 ? SHDEG * SHDEG + 3 * BINS : 2 * SHDEG * SHDEG + BINS;
   constexpr int NENC = (LEVELS * F + NDIR + 15) / 16 * 16;
@@ -104,7 +109,7 @@ __global__ void __launch_bounds__(NWG * kRows, 1) k_fused_query(const __grid_con
       else
         featurize<true>(a.enc, load3(a.pos, q), load3(a.wo, q), load3(a.nrm, q), a.rough[q], x);
     }
-    encode_row<F, LEVELS, MODE, SHDEG, BINS, SMOOTH, true, true>(a, x, A, t);
+    encode_row<F, LEVELS, MODE, SHDEG, BINS, SMOOTH, true, true, AHEAD>(a, x, A, t);
     tc::fence_proxy_async();
     tc::fence_before_sync();
     ok = bar_red_and(1 + wg, kRows, ok);
@@ -578,8 +583,10 @@ static size_t smem_bytes_for(uint32_t w_bytes) {
 template <int F, int LEVELS, int MODE, int SHDEG, int BINS, int K, int NOUTMAX, bool SMOOTH, int NWG>
 static nmg_status launch_query_nwg(const FusedArgs& a, cudaStream_t st) {
   auto kern = k_fused_query<F, LEVELS, MODE, SHDEG, BINS, K, NOUTMAX, SMOOTH, NWG>;
-  if constexpr (K == 16)
+  if constexpr (K == 16) {
     if (!a.raw && !a.raw_mode) kern = k_fused_query<F, LEVELS, MODE, SHDEG, BINS, K, NOUTMAX, SMOOTH, NWG, true>;
+    if (a.raw_mode) kern = k_fused_query<F, LEVELS, MODE, SHDEG, BINS, K, NOUTMAX, SMOOTH, NWG, false, false>;
+  }
   const size_t smem = smem_bytes_for<F, LEVELS, MODE, SHDEG, BINS, NWG>(a.w_bytes);
   nmg_status s = ensure_smem(reinterpret_cast<const void*>(kern), smem);
   if (s != NMG_OK) return s;

