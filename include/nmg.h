@@ -362,7 +362,8 @@ nmg_status nmg_network_vjp(nmg_ctx* ctx, const float* x, const float* draw, int 
  * two threads per query splitting the lobes (queries that return raw outputs
  * fall back to 4); for 16-lobe networks encoder, MLP and mixture warpgroups,
  * four threads per query in the mixture. 8-12 select warp-specialised kernels:
- * 12 encoder, MLP and mixture warpgroups, 8 (8-lobe networks) warpgroups that
+ * 12 encoder, MLP and mixture warpgroups (with five hidden layers and more the
+ * kernel of 8, but for small launches), 8 (8-lobe networks) warpgroups that
  * encode and run the MLP, and mixture warpgroups; in the others (and 8 at 16
  * lobes: 4 + 2 warpgroups, 4 slots) encoder warpgroups feed MLP + mixture
  * warpgroups through a shared-memory ring (9: 5 + 1, 5 slots; 10: 6 + 2, 6

@@ -979,6 +979,26 @@ static nmg_status launch_roles(const FusedArgs& a, cudaStream_t st) {
   return launch_roles_kernel<F, LEVELS, MODE, SHDEG, BINS, K, NOUTMAX, SMOOTH, Cfg, false>(a, grid, st);
 }
 
+// Whether the one MLP warpgroup of the three roles would bound a launch: deep
+// networks beyond the launches whose tiles the encoders share. The two roles run
+// the MLP in four warpgroups. us, three roles / two, the hash-grid network (with
+// half the levels to gather, the two roles hold at six layers on any size):
+//   hidden layers      4            5            6            7
+//   query 2,000,000    590 / 599    642 / 620    704 / 654    761 / 675
+//   pdf   2,000,000    581 / 585    627 / 606    693 / 640    748 / 660
+//   pdf   100,001       48 / 44      50 / 46      57 / 48      60 / 50
+//   raw   2,000,000    612 / 659    618 / 681    698 / 717    764 / 740
+//   raw   500,000      165 / 173    169 / 179    190 / 188    207 / 195
+static bool roles_mlp_bound(const FusedArgs& a) {
+  const long tiles = (long(a.n_max) + kRows - 1) / kRows, per_sm = (tiles + sm_count() - 1) / sm_count();
+  const int hidden = a.n_layers - 1;
+  if (per_sm <= kShareTiles) return false;
+  // A query takes the same kernel whether it returns its raw outputs or not, so that it gives the same
+  // bits (returned, three roles / two: 699 / 718 at five layers, 743 / 757 at six, 797 / 781 at seven).
+  if (!a.raw_mode) return hidden >= 5;
+  return hidden >= 7 || (hidden == 6 && (a.enc.levels <= 8 || per_sm <= 32));
+}
+
 template <int F, int LEVELS, int MODE, int SHDEG, int BINS, int K, int NOUTMAX, bool SMOOTH>
 static nmg_status launch_ws_tiling(int tiling, const FusedArgs& a, cudaStream_t st) {
   switch (tiling) {
@@ -986,7 +1006,9 @@ static nmg_status launch_ws_tiling(int tiling, const FusedArgs& a, cudaStream_t 
     case 9: return launch_ws<F, LEVELS, MODE, SHDEG, BINS, K, NOUTMAX, SMOOTH, WsE5C1>(a, st);
     case 10: return launch_ws<F, LEVELS, MODE, SHDEG, BINS, K, NOUTMAX, SMOOTH, WsE6C2>(a, st);
     case 11: return launch_ws<F, LEVELS, MODE, SHDEG, BINS, K, NOUTMAX, SMOOTH, WsE4C2S8>(a, st);
-    case 12: return launch_roles<F, LEVELS, MODE, SHDEG, BINS, K, NOUTMAX, SMOOTH, WsE4X2G1>(a, st);
+    case 12:
+      if (roles_mlp_bound(a)) return launch_duo<F, LEVELS, MODE, SHDEG, BINS, K, NOUTMAX, SMOOTH, WsN4X2G1>(a, st);
+      return launch_roles<F, LEVELS, MODE, SHDEG, BINS, K, NOUTMAX, SMOOTH, WsE4X2G1>(a, st);
   }
   return set_error(NMG_ERR_INVALID_ARG, "tiling %d is not a warp-specialised one", tiling);
 }
