@@ -48,6 +48,15 @@ inline nmg_status ensure_smem(const void* kern, size_t bytes) {
   return NMG_OK;
 }
 
+// Shared memory that a block of the current device may have (ensure_smem's limit).
+inline size_t smem_optin() {
+  int dev = 0, optin = 0;
+  cudaGetDevice(&dev);
+  if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess || optin <= 0)
+    optin = 227 << 10;
+  return size_t(optin);
+}
+
 // Number of SMs of the current device (looked up once per device).
 inline int sm_count() {
   static std::mutex mu;

@@ -358,8 +358,10 @@ NMG_D void plain_scatter(const PlainNet& p, int l, const float (&pos)[3], const 
 // input only the grid columns have parameters below. The product warps carry
 // one tile's delta from the last layer to the first in D and leave its grid
 // gradient in G; the other warps meanwhile scatter the last tile's grid
-// gradient and read the next tile's dL/draw (both buffers are double).
-template <int F>
+// gradient and read the next tile's dL/draw. D is double, and so is G where
+// shared memory holds it beside the weights; with one G (ONE_G) the product
+// warps wait for the last tile's scatter before they write theirs.
+template <int F, bool ONE_G>
 __global__ void __launch_bounds__(kPlainThreads, 2) k_plain_backward(const __grid_constant__ PlainBwd a) {
   extern __shared__ __align__(16) float sm[];
   const PlainNet& p = a.net;
@@ -376,8 +378,8 @@ __global__ void __launch_bounds__(kPlainThreads, 2) k_plain_backward(const __gri
   }
   const int d_floats = (nout > kWidth ? nout : kWidth) * kPlainRows;
   float* D = sm + w_floats;              // two buffers
-  float* G = D + 2 * d_floats;           // two buffers of [ng][64]
-  float* xs = G + 2 * ng * kPlainRows;   // two buffers of [3][64]
+  float* G = D + 2 * d_floats;           // two buffers (ONE_G: one) of [ng][64]
+  float* xs = G + (ONE_G ? 1 : 2) * ng * kPlainRows;  // two buffers of [3][64]
   const int n = plain_count(p), ni = p.enc.n_input;
   const bool mover = threadIdx.x >= kProduct;
   const int t = int(threadIdx.x) - kProduct;  // of a mover
@@ -411,7 +413,7 @@ __global__ void __launch_bounds__(kPlainThreads, 2) k_plain_backward(const __gri
     for (int l = t / (2 * kPlainRows); l < p.enc.levels; l += kMovers / (2 * kPlainRows)) {
       float g[F];
 #pragma unroll
-      for (int f = 0; f < F; ++f) g[f] = G[(buf * ng + l * F + f) * kPlainRows + r];
+      for (int f = 0; f < F; ++f) g[f] = G[((ONE_G ? 0 : buf * ng) + l * F + f) * kPlainRows + r];
       plain_scatter<F>(p, l, pos, g, t & 1u, a.gtable, a.wide != 0);
     }
   };
@@ -435,11 +437,12 @@ __global__ void __launch_bounds__(kPlainThreads, 2) k_plain_backward(const __gri
       bar_product();
       Wl += p.out[l] * kWidth;
     }
+    if (ONE_G) asm volatile("bar.sync 3, %0;" ::"n"(kPlainThreads) : "memory");  // the last tile's G has been read
     for (int c0 = tl.col; c0 < ng; c0 += kWidth) {
       plain_product(d + tl.row, Wl + c0, ng, kWidth, acc);
 #pragma unroll
       for (int c = 0; c < 8; ++c)
-        *reinterpret_cast<float4*>(G + (buf * ng + c0 + c) * kPlainRows + tl.row) =
+        *reinterpret_cast<float4*>(G + ((ONE_G ? 0 : buf * ng) + c0 + c) * kPlainRows + tl.row) =
             make_float4(acc[c][0], acc[c][1], acc[c][2], acc[c][3]);
     }
   };
@@ -452,6 +455,7 @@ __global__ void __launch_bounds__(kPlainThreads, 2) k_plain_backward(const __gri
       deltas(tile, buf);
     } else {
       if (last >= 0) scatter(last, buf ^ 1);
+      if (ONE_G) asm volatile("bar.arrive 3, %0;" ::"n"(kPlainThreads) : "memory");
       bar_movers();  // xs[buf ^ 1] is rewritten only when every lane has read it
       if (tile + int(gridDim.x) < tiles) read(tile + gridDim.x, buf ^ 1);
     }
@@ -645,9 +649,13 @@ nmg_status plain_forward(nmg_ctx* c, const nmg_shading* in, const float* x, cons
   return set_error(NMG_ERR_UNSUPPORTED, "grid_features=%d", e.feats);
 }
 
-template <int F>
-static nmg_status launch_backward(const PlainBwd& a, size_t smem, cudaStream_t st) {
-  auto kern = k_plain_backward<F>;
+// One grid-gradient buffer where two exceed what a block may have: 16 lobes with
+// selection on seven hidden layers from 81 grid columns on, the widest of the
+// others (259,584 bytes at most, the device allows 232,448; one buffer: 226,816).
+template <int F, bool ONE_G = false>
+static nmg_status launch_backward(const PlainBwd& a, size_t smem, size_t g_bytes, cudaStream_t st) {
+  if (!ONE_G && smem > smem_optin()) return launch_backward<F, true>(a, smem - g_bytes, g_bytes, st);
+  auto kern = k_plain_backward<F, ONE_G>;
   NMG_TRY(ensure_smem(reinterpret_cast<const void*>(kern), smem));
   kern<<<plain_grid(a.net.n_max), kPlainThreads, smem, st>>>(a);
   return check_launch("k_plain_backward");
@@ -674,12 +682,12 @@ nmg_status plain_backward(nmg_ctx* c, const float* x, const int* d_count, int n_
   const int ng = (a.net.n_grid + 15) / 16 * 16, dw = L.n_out_pad > kWidth ? L.n_out_pad : kWidth;
   size_t fl = 2 * size_t(dw + ng) * kPlainRows + 6 * kPlainRows + size_t(kWidth) * ng;
   for (int l = 1; l < L.n_layers; ++l) fl += size_t(L.in[l]) * L.out[l];
-  const size_t smem = fl * sizeof(float);
+  const size_t smem = fl * sizeof(float), g_bytes = size_t(ng) * kPlainRows * sizeof(float);
   switch (c->enc.feats) {
-    case 1: NMG_TRY(launch_backward<1>(a, smem, st)); break;
-    case 2: NMG_TRY(launch_backward<2>(a, smem, st)); break;
-    case 4: NMG_TRY(launch_backward<4>(a, smem, st)); break;
-    case 8: NMG_TRY(launch_backward<8>(a, smem, st)); break;
+    case 1: NMG_TRY(launch_backward<1>(a, smem, g_bytes, st)); break;
+    case 2: NMG_TRY(launch_backward<2>(a, smem, g_bytes, st)); break;
+    case 4: NMG_TRY(launch_backward<4>(a, smem, g_bytes, st)); break;
+    case 8: NMG_TRY(launch_backward<8>(a, smem, g_bytes, st)); break;
     default: return set_error(NMG_ERR_UNSUPPORTED, "grid_features=%d", c->enc.feats);
   }
   PlainWgrad g;
