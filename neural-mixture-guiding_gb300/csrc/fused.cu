@@ -915,11 +915,16 @@ nmg_status fused_check_errors(nmg_ctx* c) {
 
 
 // ---------------------------------------------------------------- autotuner
-// Candidate CTA shapes of the fused query kernel: 4, 5 or 6 warpgroups
-// (128-query tiles) per CTA, one CTA per SM. More warpgroups hide more
-// gather and MMA latency but cap registers (128, 102, 85 per thread).
+// Candidate tilings of the query (nmg_set_query_tiling): the one-pipeline
+// kernel with 4, 5 or 6 warpgroups per CTA, the paired one, the
+// warp-specialised ones. The others have no kernel for 16 lobes, whose output
+// row takes 80 columns of TMEM.
 static const int kTileCandidates[] = {4, 5, 6, 7, 8, 9, 10, 11, 12};
-static const int kTileCandidatesK16[] = {4, 7, 8};  // 128 TMEM columns per warpgroup
+static const int kTileCandidatesK16[] = {4, 7, 8};
+// Part of the cache's key: raised whenever an id comes to mean another kernel,
+// so that a winner which other kernels were timed for is not applied. (2: ids 7
+// at 16 lobes, 8 and 12; 3: 12 on deep networks.)
+constexpr int kTilingTable = 3;
 
 static std::string tune_cache_path() {
   const char* p = getenv("NMG_TUNE_CACHE");
@@ -934,8 +939,8 @@ static std::string tune_key(nmg_ctx* c, int n) {
   int bucket = 0;
   while ((1 << (bucket + 1)) <= n) ++bucket;  // log2 size class
   char buf[384];  // the device name alone can take 256 bytes
-  snprintf(buf, sizeof(buf), "%s|sm%d%d|preset%d|fp16=%d|n2^%d", prop.name, prop.major, prop.minor, fstate(c)->preset,
-           c->cfg.path == NMG_PATH_FP16, bucket);
+  snprintf(buf, sizeof(buf), "%s|sm%d%d|preset%d|h%d|fp16=%d|n2^%d|t%d", prop.name, prop.major, prop.minor,
+           fstate(c)->preset, c->cfg.hidden_layers, c->cfg.path == NMG_PATH_FP16, bucket, kTilingTable);
   for (char* q = buf; *q; ++q)
     if (*q == ' ') *q = '_';
   return buf;
