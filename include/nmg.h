@@ -242,7 +242,7 @@ nmg_status nmg_reserve(nmg_ctx* ctx, int max_queries, int max_batch);
 
 /* Device bytes the field holds: parameters, optimiser state, weight copies
  * and workspaces. The FP32 path stores each layer's activations of a
- * training batch (about 1.9 KB per record for the hash-grid network); the
+ * training batch (about 2.5 KB per record for the hash-grid network); the
  * BF16/FP16 paths recompute them inside the fused training kernel, so their
  * footprint does not grow with max_batch. No reference counterpart (tcnn
  * allocates every layer's forward activations per training call,

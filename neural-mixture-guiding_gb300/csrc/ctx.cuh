@@ -26,12 +26,12 @@ struct Layout {
 struct Workspace {
   int cap_q = 0, cap_b = 0;
   // plain path
-  float* x = nullptr;      // [cap][n_input]
+  float* x = nullptr;      // [cap_b][n_input] rows of a batch (nmg_train_frame)
   // kept for the plain backward pass, in tiles of [column][kPlainRows rows]
   float* enc = nullptr;    // n_enc_pad columns
   float* h[kMaxLayers] = {};  // 64 columns: activations after ReLU
   float* delta[kMaxLayers] = {};  // each layer's output columns: dL/d(output before ReLU)
-  float* raw = nullptr;    // [cap][n_out_pad]
+  float* raw = nullptr;    // [max(cap_q, cap_b)][n_out_pad]
   float* draw = nullptr;   // [cap_b][n_out_pad]
   double* partials = nullptr;  // block partial sums (loss, grad norm)
   int n_partials = 0;

@@ -707,7 +707,6 @@ nmg_status pack_images(nmg_ctx* c, cudaStream_t st) {
 static void plan_cells(const nmg_ctx* c, FusedState& s) {
   const EncodingParams& e = c->enc;
   CellPackArgs& p = s.cells;
-  p.feats = e.feats;
   for (int l = 0; l < e.levels; ++l) {
     const uint32_t T = e.offset[l + 1] - e.offset[l];
     const unsigned long long r = e.res[l];

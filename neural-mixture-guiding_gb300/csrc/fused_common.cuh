@@ -777,7 +777,7 @@ struct PackArgs {
 // level i of the n_lvl packed ones has entries [first[i], first[i + 1]) of the
 // running record count.
 struct CellPackArgs {
-  int n_lvl, feats;
+  int n_lvl;
   uint32_t first[kMaxLevels + 1];
   uint32_t T[kMaxLevels], res[kMaxLevels], table_off[kMaxLevels], cell_off[kMaxLevels];
   uint32_t oct_mask;  // bit i: packed level i has 8-corner records

@@ -156,9 +156,10 @@ static nmg_status reserve(nmg_ctx* c, int max_q, int max_b) {
   max_b = max_b > w.cap_b ? max_b : w.cap_b;
   cudaDeviceSynchronize();
   free_workspace(c);
-  // The FP32 path stores every layer's activations of a batch for its
-  // backward; the fused paths recompute them inside the training kernel and
-  // keep only the query-side input rows and raw outputs (for nmg_pdf).
+  // The FP32 path keeps the raw outputs between its kernels, every layer's
+  // activations and deltas of a batch for its backward, and the input rows and
+  // records of a batch that nmg_train_frame gathers; the fused paths keep all of
+  // these on chip.
   const bool fp32 = c->cfg.path == NMG_PATH_FP32;
   const int cap = fp32 && max_b > max_q ? max_b : max_q;
   const Layout& L = c->lay;
@@ -169,13 +170,13 @@ static nmg_status reserve(nmg_ctx* c, int max_q, int max_b) {
     if ((s = dalloc(&(p), (n))) != NMG_OK) return s; \
     w.bytes += size_t(n) * sizeof(*(p));              \
   } while (0)
-  A(w.x, capz * c->enc.n_input);
   A(w.partials, 2 * 2048);
   A(w.batch_counts, kMaxFrameBatches);
-  A(w.raw, capz * L.n_out_pad);
   w.n_partials = 2 * 2048;
   if (fp32) {
+    A(w.raw, capz * L.n_out_pad);
     if (max_b > 0) {
+      A(w.x, size_t(max_b) * c->enc.n_input);
       const size_t rows = (size_t(max_b) + kPlainRows - 1) / kPlainRows * kPlainRows;
       A(w.enc, rows * c->enc.n_enc_pad);
       for (int l = 0; l < L.n_layers - 1; ++l) A(w.h[l], rows * kWidth);
