@@ -76,8 +76,10 @@ def _stream(stream):
     if stream is not None:
         return C.c_void_p(stream.cuda_stream)
     import torch
-    # the handle itself: a Stream object around it costs 3 to 5 us a call
-    return C.c_void_p(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
+    # the handle itself, where this torch has the (private) call for it: a Stream object around it
+    # costs 3 to 5 us a call
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    return C.c_void_p(raw(torch.cuda.current_device()) if raw else torch.cuda.current_stream().cuda_stream)
 
 
 def mixture_opts(n_lobes, stride, kappa_softplus=False, kappa_poly=True, selection=False):
