@@ -33,23 +33,6 @@ struct EncodingParams {
   float inv_size[3];  // 1 / size of the inflated box
 };
 
-// grid.h:171-187 with the coherent-prime hash (grid.h:132-135).
-NMG_D uint32_t grid_index(int hash, uint32_t T, uint32_t res, uint32_t x, uint32_t y, uint32_t z) {
-  uint32_t stride = 1, index = 0;
-  const uint32_t p[3] = {x, y, z};
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    if (stride <= T) {
-      index += p[d] * stride;
-      stride *= res;
-    }
-  }
-  if (hash && T < stride) index = (x * 1u) ^ (y * 2654435761u) ^ (z * 805459861u);
-  return index % T;
-}
-
-// common_device.h:484-495 (pos_fract) without FMA contraction so the cell
-// index matches the host computation bit for bit.
 NMG_D f3 unit3f(f3 a) {
   const float n2 = dot3(a, a);
   if (!(n2 > 0.f)) return a;
@@ -57,42 +40,14 @@ NMG_D f3 unit3f(f3 a) {
   return f3{a.x * r, a.y * r, a.z * r};
 }
 
+// common_device.h:484-495 (pos_fract) without FMA contraction so the cell
+// index matches the host computation bit for bit.
 NMG_D void pos_fract(float x, float scale, int smooth, float* w, uint32_t* g) {
   float p = __fadd_rn(__fmul_rn(x, scale), 0.5f);
   float fl = floorf(p);
   *g = uint32_t(int(fl));
   float f = p - fl;
   *w = smooth ? f * f * (3.f - 2.f * f) : f;
-}
-
-// Corner c of the level's cell around `pos`: entry index into the table and
-// trilinear weight.
-struct Corners {
-  uint32_t g[3];
-  float w[3];
-};
-
-NMG_D void level_cell(const EncodingParams& e, int l, const float* pos, Corners& c) {
-#pragma unroll
-  for (int d = 0; d < 3; ++d) pos_fract(pos[d], e.scale[l], e.smoothstep, &c.w[d], &c.g[d]);
-}
-
-NMG_D void corner(const EncodingParams& e, int l, const Corners& c, int k, uint32_t* entry, float* weight) {
-  float wt = 1.f;
-  uint32_t p[3];
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    if ((k & (1 << d)) == 0) {
-      wt *= 1.f - c.w[d];
-      p[d] = c.g[d];
-    } else {
-      wt *= c.w[d];
-      p[d] = c.g[d] + 1;
-    }
-  }
-  const uint32_t T = e.offset[l + 1] - e.offset[l];
-  *entry = e.offset[l] + grid_index(e.grid_hash, T, e.res[l], p[0], p[1], p[2]);
-  *weight = wt;
 }
 
 // spherical_harmonics.h:46-85: real SH basis of (x, y, z) up to degree 4.

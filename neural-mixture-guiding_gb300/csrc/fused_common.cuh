@@ -265,7 +265,7 @@ NMG_D void cell_features(const FusedArgs& a, int l, const uint32_t (&g)[3], cons
 // Features of grid level l at position p3 (F values into out). The cell and
 // weights follow grid.h:221-385; the corner indices are formed from per-axis
 // terms (x, y*P1, z*P2 for hashed levels, x, y*res, z*res^2 for dense ones),
-// which equal grid_index's value for every corner, and the corner weight is
+// which equal grid.h:171-187's index for every corner, and the corner weight is
 // (w_x' * w_y') * w_z' as in the reference. PAIR (F = 2): the x and x+1
 // corners of a (y, z) pair that share an aligned 8-byte word (every other
 // cell: for dense levels e1 = e0 + 1, for hashed ones e1 = e0 ^ 1 when x is

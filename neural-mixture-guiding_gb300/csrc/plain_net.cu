@@ -70,7 +70,8 @@ NMG_D int plain_count(const PlainNet& p) {
   return n < 0 ? 0 : (n > p.n_max ? p.n_max : n);
 }
 
-// grid_index with the level's strides and hashing worked out on the host.
+// Entry of a corner (grid.h:171-187 with the coherent-prime hash, grid.h:132-135),
+// the level's strides and hashing worked out on the host (plain_net).
 NMG_D uint32_t plain_index(const PlainNet& p, int l, uint32_t x, uint32_t y, uint32_t z) {
   const uint32_t T = p.T[l];
   const uint32_t i = (p.hashed >> l) & 1u ? x ^ (y * 2654435761u) ^ (z * 805459861u)
@@ -583,7 +584,7 @@ static PlainNet plain_net(const nmg_ctx* c, const float* weights, const int* d_c
     p.w[l] = weights + c->lay.off[l];
   }
   p.table = weights + c->lay.n_mlp;
-  for (int l = 0; l < c->enc.levels; ++l) {  // grid_index's strides (grid.h:171-187)
+  for (int l = 0; l < c->enc.levels; ++l) {  // strides and hashing as grid.h:171-187
     const uint32_t T = c->enc.offset[l + 1] - c->enc.offset[l];
     uint32_t s[3] = {0, 0, 0}, stride = 1;
     for (int d = 0; d < 3; ++d)
