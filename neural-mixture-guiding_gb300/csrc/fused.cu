@@ -167,16 +167,14 @@ __global__ void __launch_bounds__(NWG * kRows, 1) k_fused_query(const __grid_con
   }
 }
 
-// Tiling 7 of the 8-lobe networks: two pipelines per CTA, each two warpgroups on one 128-query tile
-// (the layout of the training kernel): warps w and w + 4 read the same TMEM
-// lane quadrant, so every query has two threads, which split the encoding's
-// grid levels, each hidden epilogue's columns and the mixture's lobes. With
-// K / 2 lobes per thread the lobes stay in registers from activation to pdf
-// (one pass, where one thread holding all 16 re-derives them from TMEM);
-// the lobe-weight total, the selection scan (continued by the second half
-// where the first half's lobes ran out, the reference's sequential
-// subtraction), the sampled lobe and the pdf's partial sums cross between
-// the two through shared memory. Queries without raw outputs only.
+// Tiling 7 of the 8-lobe networks: two pipelines per CTA, each two warpgroups
+// on one 128-query tile (the layout of the training kernel): warps w and w + 4
+// read the same TMEM lane quadrant, so every query has two threads, which split
+// the encoding's grid levels, each hidden epilogue's columns and the mixture's
+// lobes; the lobe-weight total, the selection scan (continued by the second half
+// where the first half's lobes ran out, the reference's sequential subtraction),
+// the sampled lobe and the pdf's partial sums cross between the two through
+// shared memory. Queries without raw outputs only.
 template <int F, int LEVELS, int MODE, int SHDEG, int BINS, int K, int NOUTMAX, bool SMOOTH>
 __global__ void __launch_bounds__(4 * kRows, 1) k_fused_query_pair(const __grid_constant__ FusedArgs a) {
   constexpr int NP = 2, KH = K / 2;

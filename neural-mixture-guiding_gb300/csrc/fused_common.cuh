@@ -183,7 +183,13 @@ NMG_D void load_feats(const uint16_t* table, uint32_t entry, float* v, bool fp16
 // Levels get records from the coarsest on while they fit kCellBytes per copy
 // of the table: for the hash-grid network levels 0-2 (32-byte) and 3 (16-byte)
 // of its five dense levels, 3.7 MB for each of the training and the inference
-// table, for the reference network six of eight.
+// table, for the reference network six of eight (4.2 MB). The line lies where a
+// context with the default table still holds less than 28 bytes a parameter and
+// 8 MB. us without records / with these / with a budget of 10 MB, which takes in
+// the hash grid's fifth dense level (5.5 MB more a copy; the reference network's
+// seventh would be 7.3 MB): 2,073,600 queries 688 / 538 / 523, 900,000 at 16 lobes
+// 348 / 320 / 315, the reference network's pdf of 550,001 134 / 110 / 110, training
+// steps of 262,144 and 65,536 records 376 / 373 / 371 and 246 / 249 / 249.
 constexpr size_t kCellBytes = 4608u << 10;
 constexpr uint32_t kOctEntries = 1u << 16;  // F = 2 levels up to this size have 32-byte records
 
@@ -269,10 +275,8 @@ NMG_D void cell_features(const FusedArgs& a, int l, const uint32_t (&g)[3], cons
 // (w_x' * w_y') * w_z' as in the reference. PAIR (F = 2): the x and x+1
 // corners of a (y, z) pair that share an aligned 8-byte word (every other
 // cell: for dense levels e1 = e0 + 1, for hashed ones e1 = e0 ^ 1 when x is
-// even) are read with one 8-byte load -- a quarter fewer L1 requests: the
-// query kernels take 648 instead of 678 us (warp-specialised) and 797
-// instead of 834 us (one pipeline per warpgroup), the training step 0.492
-// instead of 0.499 ms.
+// even) are read with one 8-byte load: a quarter fewer L1 requests, 4% of the
+// query kernels' time and 1.5% of the training step's when it came in.
 template <int F, bool SMOOTH, bool PAIR = false>
 NMG_D void grid_level(const FusedArgs& a, int l, const float (&p3)[3], float* out) {
   float w[3];
@@ -614,10 +618,12 @@ NMG_D f3 face_fwd(f3 n, f3 v) { return dot3(n, v) > 0.f ? n : f3{-n.x, -n.y, -n.
 // optional raw row, then (unless raw_mode) the mixture with the optional
 // cosine lobe, and either the sampled direction with its pdf, lobe and
 // selection probability, or (a.wi set) the pdf at the given direction.
-// (The direction is stored per thread here: gathering a warp's directions
-// into whole-sector float4 stores, as the 16-lobe epilogues do, kept three
-// more values live across the pdf and made the 8-lobe consumers spill:
-// query pass 0.647 -> 0.751 ms.)
+// (The direction is stored per thread here, as the kernels with mixture
+// warpgroups of their own do: gathering a warp's directions into whole-sector
+// float4 stores, as query_epilogue_streamed does, kept three more values live
+// across the pdf and made the consumers spill. To mapped host memory the scalar
+// stores cost nothing that shows: nmg_query_host at 16 lobes, 500,000 queries,
+// 193 us, the device call 185.)
 template <int K, int NOUTMAX>
 NMG_D void query_epilogue(const FusedArgs& a, long q, const float (&r)[NOUTMAX]) {
   if (a.raw) {

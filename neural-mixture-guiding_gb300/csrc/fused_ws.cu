@@ -11,8 +11,9 @@
 // Here the roles are split inside one persistent CTA per SM. Three kernels:
 //   * k_fused_query_roles (the default of the hash-grid networks): encoders,
 //     an MLP warpgroup, mixture warpgroups;
-//   * k_fused_query_duo (the default of the reference network): warpgroups
-//     that encode and run the MLP, mixture warpgroups;
+//   * k_fused_query_duo (the default of the reference network and of deep 8-lobe
+//     ones, roles_mlp_bound): warpgroups that encode and run the MLP, mixture
+//     warpgroups;
 //   * k_fused_query_ws (tilings 9-11 and the 16-lobe tiling 8): E encoder
 //     warpgroups, and C consumer warpgroups that run the MLP and the mixture.
 // In the last, thread t of an encoder warpgroup writes row t of a 128-query
@@ -428,7 +429,12 @@ NMG_D void store_raw16(const FusedArgs& a, long q, int c16, const float (&r)[16]
 // a thread's gathers run on from level to level) and shared, 8 / 16 lobes, us:
 // 4,999 queries 17.0 / 17.2 and 14.1 / 14.6; 38,912 (2 tiles per SM) 23.7 / 27.8
 // and 21.3 / 23.4; 77,824 (4 tiles) 36.9 / 43.8 and 36.2 / 39.9; 120,000 52.3 / 64.4
-// and 55.3 / 66.8.
+// and 55.3 / 66.8. The line is drawn on the launch's capacity: with both forms in one
+// kernel, chosen by the device count, the encoders spill (2,073,600 queries 548
+// instead of 538 us, 900,000 at 16 lobes 330 instead of 319). So 16 lobes with a
+// count of one to two tiles per SM below a larger capacity take 27.5 us, as one
+// tile's mixture follows the other's (shared 25.0, the kernel before the roles 25.1);
+// every other count is faster than with that kernel.
 constexpr int kShareTiles = 4;
 template <int E_, int X_, int G_, int RE_, int RM_, int RX_>
 struct WsRoles {

@@ -8,10 +8,13 @@
 // a tile of 64 rows in shared memory from the first layer to the last, next to
 // all of the weights. Four warps of a block do the matrix products of one tile
 // while the other four gather the next tile's table entries (forward) or
-// scatter the last tile's grid gradient (backward); two blocks per SM. A
-// product thread holds 4 rows x 8 columns, three 16-byte shared loads per 32
-// FMAs. The forward kernel takes 409 us for the queries above, bound by the
-// products' shared loads (472 us with 4 x 4 per thread on all eight warps and
+// scatter the last tile's grid gradient (backward). Two blocks fit an SM at
+// three hidden layers and up to 8 lobes (92 KB forward for the reference
+// network, 104 KB backward for the hash-grid one); 16 lobes (119 and 118 KB) and
+// deeper networks run one. A product thread holds 4 rows x 8 columns, three
+// 16-byte shared loads per 32 FMAs. The forward kernel takes 410 us for 524,288
+// queries of the reference network, bound by issue slots that FMAs (48% of them
+// busy) share with the products' shared loads (472 us with 4 x 4 per thread on all eight warps and
 // the roles one after the other, the shared-memory pipe 80% busy; 493 us at 2
 // rows x 16 columns, 444 us with eight gathering warps, 430 us on 128-row
 // tiles at 8 x 4).
