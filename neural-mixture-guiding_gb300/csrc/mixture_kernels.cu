@@ -217,6 +217,41 @@ __global__ void __launch_bounds__(kThreads, K <= 8 ? 8 : 1) k_mixture_pdf2(const
   }
 }
 
+// The same pdf with the lobes kept, each weight normalised before it meets its
+// density, for a row with a concentration beyond kKappaLean, where lambda times
+// the normaliser leaves FP32's range (a softplus of a raw output as large; the
+// clamped exponential ends at e^15). Of the product with the cosine lobe, the
+// exponent's cosines are held to 1: a mean that rounds to a length above 1 would
+// make it infinite here.
+constexpr float kKappaLean = 1e30f;
+template <int K, bool COS>
+__device__ __noinline__ float pdf_kept(const float* row, f3 w, f3 mb, float nb) {
+  Mix<K> m;
+  mix_activate<K, kMixFast, kAngTab>(m, row, 1);
+  if (COS) {
+    float total = 0.f;
+    for (int i = 0; i < K; ++i) {
+      const float ka = m.kap[i], kb = kCosineKappa;
+      const f3 ma = m.mu[i];
+      f3 nm = add3(scale3(ma, ka), scale3(mb, kb));
+      const float n2 = dot3(nm, nm), rn = rsqrtf(n2);
+      const bool some = n2 * rn >= 1e-3f;
+      nm = some ? scale3(nm, rn) : ma;
+      const float nk = some ? n2 * rn : 0.f;
+      const float e = xexp<kMixFast>(ka * fminf(0.f, dot3(nm, ma) - 1.f) + kb * fminf(0.f, dot3(nm, mb) - 1.f));
+      const float pk = prod_norm<kMixFast>(nk), pa = ka < 1e-3f ? NMG_INV_4PI : m.nrm[i];
+      m.lam[i] *= xdiv<kMixFast>(pa * nb, pk) * e;
+      m.kap[i] = nk;
+      m.mu[i] = nm;
+      m.nrm[i] = pk;
+      total += m.lam[i];
+    }
+    const float inv = 1.f / fmaxf(total, NMG_EPS);
+    for (int i = 0; i < K; ++i) m.w[i] = m.lam[i] * inv;
+  }
+  return mix_pdf<K, kMixFast>(m, w);
+}
+
 // The other pdfs (with the cosine lobe, or odd K): one thread per query sums
 // its lobes one after the other and keeps none, so that 8 blocks fit an SM.
 // Instruction issue and the special-function unit bound it. 300,001 queries at
@@ -237,7 +272,14 @@ __global__ void __launch_bounds__(kThreads, 8) k_mixture_pdf(const float* __rest
     float total = 0.f, p = 0.f;
 #pragma unroll
     for (int i = 0; i < K; ++i) lobe_pdf_lean<COS>(row[i], kappa_softplus, w, mb, nb, &total, &p);
-    pdf[q] = p / (COS ? fmaxf(total, NMG_EPS) : total);  // distribution.h:191
+    p /= COS ? fmaxf(total, NMG_EPS) : total;  // distribution.h:191
+    if (kappa_softplus) {
+      bool beyond = false;
+#pragma unroll 1
+      for (int i = 0; i < K; ++i) beyond |= row[i].y > kKappaLean;
+      if (beyond) p = pdf_kept<K, COS>(raw + q * stride, w, mb, nb);
+    }
+    pdf[q] = p;
   }
 }
 
