@@ -433,6 +433,11 @@ NMG_D float prod_norm_flat(float k) {
   return k < 1e-3f ? NMG_INV_4PI : v;
 }
 constexpr float kCosineKappa = 2.18853f;  // distribution.h:184-195
+// Squared lengths are held to this before rsqrt_ftz: below 1e-38 it would take
+// them for 0 and return an infinite factor for a length that is not 0 (a softplus
+// concentration below 1e-19 beside a normal of zeros). Lengths that matter (1e-3
+// and up) are far above.
+constexpr float kTinySquare = 1e-30f;
 
 // lobe_cosine<true> without branches, its sum of scaled means fused in a stated
 // order, so that a lobe's mean and weight are the same bit for bit whatever
@@ -447,7 +452,7 @@ NMG_D void lobe_cosine_flat(f3 mb, float nb, float& lam, float& kap, f3& mu, flo
   f3 nm = LOBE_FIRST ? f3{fmaf(ma.x, ka, mb.x * kb), fmaf(ma.y, ka, mb.y * kb), fmaf(ma.z, ka, mb.z * kb)}
                      : f3{fmaf(mb.x, kb, ma.x * ka), fmaf(mb.y, kb, ma.y * ka), fmaf(mb.z, kb, ma.z * ka)};
   const float n2 = dot3(nm, nm);
-  const float rn = rsqrt_ftz(n2);
+  const float rn = rsqrt_ftz(fmaxf(n2, kTinySquare));
   float nk = n2 * rn;
   const bool some = nk >= 1e-3f;
   nm = f3{some ? nm.x * rn : ma.x, some ? nm.y * rn : ma.y, some ? nm.z * rn : ma.z};
@@ -752,7 +757,7 @@ NMG_D void lobe_pdf_lean(float4 r, int kappa_softplus, f3 wi, f3 mb, float nb, f
   }
   const float kb = kCosineKappa;
   f3 nm{fmaf(ma.x, ka, mb.x * kb), fmaf(ma.y, ka, mb.y * kb), fmaf(ma.z, ka, mb.z * kb)};
-  const float n2 = dot3_fma(nm, nm), rn = rsqrt_ftz(n2);
+  const float n2 = dot3_fma(nm, nm), rn = rsqrt_ftz(fmaxf(n2, kTinySquare));
   const bool some = n2 * rn >= 1e-3f;
   const float nk = some ? n2 * rn : 0.f;
   nm = f3{some ? nm.x * rn : ma.x, some ? nm.y * rn : ma.y, some ? nm.z * rn : ma.z};
