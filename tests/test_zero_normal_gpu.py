@@ -29,17 +29,16 @@ def test_mixture_kernels(nmg, K):
     assert float((q / UNIFORM - 1).abs().max()) <= 1e-5
 
 
-@pytest.mark.parametrize("tiling", [0, 4, 7, 8, 9, 12])
-@pytest.mark.parametrize("net", [(0, 1, 8), (1, 1, 8), (1, 2, 16), (1, 0, 16)], ids=["reference", "hash", "hash-K16", "fp32"])
-def test_queries(nmg, net, tiling):
+NETS = [((0, 1, 8), (0, 4, 7, 8, 9, 12)), ((1, 1, 8), (0, 4, 7, 8, 9, 12)), ((1, 2, 16), (0, 4, 7, 8)), ((1, 0, 16), (0,))]
+
+
+@pytest.mark.parametrize("preset,path,lobes,tiling", [net + (t,) for net, tilings in NETS for t in tilings])
+def test_queries(nmg, preset, path, lobes, tiling):
     import torch
-    preset, path, lobes = net
     n = 20000
     f = nmg.GuidingField(nmg.config(preset, path=path, n_lobes=lobes, kappa_softplus=1), max_queries=n, max_batch=0)
     try:
         if tiling:
-            if path == 0 or (lobes == 16 and tiling in (9, 12)):
-                pytest.skip("no such kernel")
             f.set_query_tiling(tiling)
         g = torch.Generator(device="cuda")
         g.manual_seed(4)
