@@ -185,7 +185,7 @@ NMG_D void load_feats(const uint16_t* table, uint32_t entry, float* v, bool fp16
 // of its five dense levels, 3.7 MB for each of the training and the inference
 // table, for the reference network six of eight (4.2 MB). The line lies where a
 // context with the default table still holds less than 28 bytes a parameter and
-// 8 MB. us without records / with these / with a budget of 10 MB, which takes in
+// 8 MB. us without records / with these / with a limit of 10 MB, which takes in
 // the hash grid's fifth dense level (5.5 MB more a copy; the reference network's
 // seventh would be 7.3 MB): 2,073,600 queries 688 / 538 / 523, 900,000 at 16 lobes
 // 348 / 320 / 315, the reference network's pdf of 550,001 134 / 110 / 110, training
